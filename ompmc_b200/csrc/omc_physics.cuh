@@ -59,6 +59,22 @@ OMC_HD double m_pow(double x, double y) { return pow(x, y); }
 OMC_HD float m_pow(float x, float y) { return powf(x, y); }
 template <typename R> OMC_HD R m_max(R a, R b) { return a > b ? a : (b == b ? b : a); }
 template <typename R> OMC_HD R m_min(R a, R b) { return a < b ? a : (b == b ? b : a); }
+// A product rounded on its own, also where the compiler would contract it
+// into a following sum.
+OMC_HD double m_mul(double a, double b) {
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+OMC_HD float m_mul(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
 template <typename R> OMC_HD R sq(R x) { return x * x; }
 template <typename R> OMC_HD bool m_abs_lt(R a, R b) { return (a < R(0) ? -a : a) < b; }
 
@@ -108,6 +124,22 @@ template <typename R>
 OMC_HD const PhBin<R> &pbin(const DevData<R> &D, int imed, int l) {
     l = l < 0 ? 0 : (l >= D_MXGE ? D_MXGE - 1 : l);
     return D.ph[imed * D_MXGE + l];
+}
+
+// Environments with kBuffered = true keep their next random numbers in a
+// buffer; rng_ensure asks them to have the next n at hand, where the lanes of
+// a warp are together.  The numbers themselves do not change.
+template <typename Env, typename = void>
+struct BufferedRng {
+    static constexpr bool value = false;
+};
+template <typename Env>
+struct BufferedRng<Env, decltype((void)Env::kBuffered)> {
+    static constexpr bool value = Env::kBuffered;
+};
+template <typename Env>
+OMC_HD void rng_ensure(Env &g, int n) {
+    if constexpr (BufferedRng<Env>::value) g.rng.ensure(n);
 }
 
 // ------------------------------------------------------------- geometry
@@ -183,17 +215,20 @@ OMC_HD R hownear(const DevData<R> &D, const Part<R> &p) {
 
 // ------------------------------------------------------------ rotations
 // Azimuth by rejection in the unit half disc (selectAzimuthalAngle,
-// ompmc.c:102-125).
+// ompmc.c:102-125).  Where each number is drawn by a branch of its own, the
+// squares end up in other basic blocks than their sums and are rounded
+// before them; with buffered numbers that has to be said.
 template <typename R, typename Env>
 OMC_HD void azimuth(Env &g, R &cphi, R &sphi) {
     R x, x2, y, y2, r2;
     int guard = 0;
     do {
+        rng_ensure(g, 3);
         x = g.uni();
         x = R(2) * x - R(1);
-        x2 = x * x;
+        x2 = BufferedRng<Env>::value ? m_mul(x, x) : x * x;
         y = g.uni();
-        y2 = y * y;
+        y2 = BufferedRng<Env>::value ? m_mul(y, y) : y * y;
         r2 = x2 + y2;
         if (++guard > 1000) { g.err(ERR_LOOP); x2 = R(1); y2 = R(0); x = R(1); y = R(0); r2 = R(1); break; }
     } while (r2 > R(1));
@@ -818,6 +853,7 @@ OMC_COLD PhotonEventOut<R> photon_event_outline(const DevData<R> &D, Part<R> p, 
 // its weight and energy are zeroed (it deposits nothing).
 template <typename R, typename Env>
 OMC_HD void roulette(const DevData<R> &D, Env &g, Part<R> &q) {
+    rng_ensure(g, 1);
     R rnno = g.uni();
     if (rnno * R(D.nsplit) > R(1)) {
         q.wt = R(0);
@@ -832,6 +868,7 @@ OMC_HD void roulette(const DevData<R> &D, Env &g, Part<R> &q) {
 // first and the second is pushed (rannih, ompmc.c:4129-4185).
 template <typename R, typename Env>
 OMC_HD void rannih(const DevData<R> &D, Env &g, Part<R> &p) {
+    rng_ensure(g, 2);
     R rnno = g.uni();
     R costhe = R(2) * rnno - R(1);
     R sinthe = m_sqrt(m_max(R(0), (R(1) - costhe) * (R(1) + costhe)));
@@ -1174,6 +1211,7 @@ OMC_HD void mscat(const DevData<R> &D, Env &g, int imed, int qel, bool &spin_ind
             R xi, rejf, rnno;
             int guard = 0;
             do {
+                rng_ensure(g, 4);
                 xi = g.uni();
                 xi = R(2) * chia2 * xi / (R(1) - xi + chia2);
                 cost = R(1) - xi;
@@ -1198,6 +1236,7 @@ OMC_HD void mscat(const DevData<R> &D, Env &g, int imed, int qel, bool &spin_ind
                 R xi, cosz, rejf, rnno;
                 int guard = 0;
                 do {
+                    rng_ensure(g, 5);
                     xi = g.uni();
                     xi = R(2) * chia2 * xi / (R(1) - xi + chia2);
                     cosz = R(1) - xi;
@@ -1250,6 +1289,7 @@ OMC_HD void mscat(const DevData<R> &D, Env &g, int imed, int qel, bool &spin_ind
         R xi, rejf, rnno;
         int guard = 0;
         do {
+            rng_ensure(g, 5);
             xi = g.uni();
             R ak = xi * R(31);
             int k = (int)ak;
@@ -1291,6 +1331,7 @@ OMC_HD void sscat(const DevData<R> &D, Env &g, int imed, int qel, R chia2, R elk
     R xi, rejf, rnno;
     int guard = 0;
     do {
+        rng_ensure(g, 4);
         xi = g.uni();
         xi = R(2) * chia2 * xi / (R(1) - xi + chia2);
         cost = R(1) - xi;
@@ -1351,6 +1392,7 @@ OMC_HD R msdist(const DevData<R> &D, Env &g, const Part<R> &p, int imed, int iq,
 #pragma unroll 1
     for (int k = 0; k < 2; k++) {
         R w, st, cp, sp;
+        rng_ensure(g, 10);
         mscat(D, g, imed, qel, spin_index, find_index, elke, beta2, xi, lambda, chia2, w, st, mi, omega2, si);
         azimuth(g, cp, sp);
         if (k == 0) {
@@ -1542,6 +1584,7 @@ OMC_HD int electron_transport(const DevData<R> &D, Env &g, Part<R> &p, R &edep_e
         // (demfp is re-drawn here), so an event can stop after a budget of
         // iterations and resume in a later launch exactly where it was.
         if (!g.tstep_take()) return E_ALIVE;
+        rng_ensure(g, 1);
         bool compute_tstep = true;
         R eke = eie - RMr;
         if (imed != -1) {
@@ -1577,6 +1620,7 @@ OMC_HD int electron_transport(const DevData<R> &D, Env &g, Part<R> &p, R &edep_e
                 nch++;
             }
             if (++guard > 20000 || !g.tick()) { g.err(ERR_LOOP); return E_DEAD; }
+            rng_ensure(g, 12);
             if (D.chsteps <= 0 && D.ref_compat) {
                 // quirk: the reference declares total_tstep inside this loop
                 // (ompmc.c:4799), so every step after the first of a tstep
@@ -1785,6 +1829,7 @@ OMC_HD int electron_transport(const DevData<R> &D, Env &g, Part<R> &p, R &edep_e
         R dedx0 = pwl(B.dedx, elke);
         sigf /= dedx0;
         R sigratio = sigf / sig0;
+        rng_ensure(g, 1);
         R rfict = g.uni();
         if (!(rfict >= sigratio)) break;
     }
