@@ -54,6 +54,9 @@ int cuda_check(omc_engine *e, cudaError_t rc, const char *what) {
                    std::string(what) + ": " + cudaGetErrorString(rc));
 }
 
+// Batch tallies of a plain run held at once, at most (bytes).
+constexpr long PLAIN_TALLIES = 1L << 30;
+
 template <typename T>
 static int upload(omc_engine *e, DBuf &b, const std::vector<T> &v) {
     int rc = b.alloc(v.size() * sizeof(T));
@@ -668,21 +671,31 @@ int omc_run_beam(omc_engine *e, const omc_beam *b, int64_t ncase, int nbatch, ui
         BeamSrc<double> S = beam_setup<double>(e, b);
         S.cdf1 = ncdf > 0 ? cdf.as<double>() : nullptr;
         S.cdf2 = ncdf > 0 ? cdf.as<double>() + ncdf : nullptr;
+        // batches run together, each on a tally of its own, as many as fit
+        // PLAIN_TALLIES bytes (one at a time where not even that can be had)
         DBuf &work = e->run_work;
-        if ((rc = work.reserve(nv * 8))) return set_err(e, rc, "device allocation for tallies failed");
-        cudaMemsetAsync(work.p, 0, nv * 8, e->stream);
+        int group = (int)std::max<long>(1, std::min<long>(nbatch, PLAIN_TALLIES / (nv * 8)));
+        while ((rc = work.reserve((size_t)group * nv * 8)) == OMC_E_NOMEM && group > 1) {
+            cudaGetLastError();
+            group = 1;
+        }
+        if (rc) return set_err(e, rc, "device allocation for tallies failed");
+        cudaMemsetAsync(work.p, 0, (size_t)group * nv * 8, e->stream);
         int block = e->opt.block > 0 ? e->opt.block : 128;
         cudaEvent_t t0, t1;
         cudaEventCreate(&t0);
         cudaEventCreate(&t1);
         cudaEventRecord(t0, e->stream);
-        for (int ib = 0; ib < nbatch; ib++) {
+        for (int b0 = 0; b0 < nbatch; b0 += group) {
+            const int nb = std::min(group, nbatch - b0);
             long nl = 0;
-            if ((rc = plain_beam_batch(e, S, work.as<double>(), seed, (long)ib * nper, nper, acc.as<double>() + 1,
-                                       block, &nl)))
+            if ((rc = plain_beam_batches(e, S, work.as<double>(), seed, (long)b0 * nper, nb, nper,
+                                         acc.as<unsigned long long>() + 2, acc.as<double>() + 1, block, &nl)))
                 return rc;
-            if ((rc = fold(e, work.as<double>(), sum.as<double>(), sum2.as<double>(), nv, 1.0))) return rc;
-            ks.launches += nl + 1;
+            for (int ib = 0; ib < nb; ib++)
+                if ((rc = fold(e, work.as<double>() + (size_t)ib * nv, sum.as<double>(), sum2.as<double>(), nv, 1.0)))
+                    return rc;
+            ks.launches += nl + nb;
         }
         cudaEventRecord(t1, e->stream);
         if ((rc = cuda_check(e, cudaEventSynchronize(t1), "beam transport"))) return rc;

@@ -98,13 +98,14 @@ namespace omc {
 int set_err(omc_engine *e, int code, const std::string &msg);
 int cuda_check(omc_engine *e, cudaError_t rc, const char *what);
 
-// Plain FP64 form (omc_plain.cu).
-// *launches (may be null) receives the kernel launches made: a batch is
-// split into launches of at most a few million histories.
-int plain_beam_batch(omc_engine *e, const BeamSrc<double> &S, double *work, uint64_t seed, long hist0, long n,
-                     double *src_energy, int block, long *launches = nullptr);
-int plain_beamlet_batch(omc_engine *e, const BeamletSrc<double> &S, int ib, double *work, uint64_t seed, long hist0,
-                        long n, int block);
+// Plain FP64 form (omc_plain.cu): nbatch batches of nper histories each from
+// history hist0 on, batch k tallied at work + k * nvox, in launches of at
+// most a few million histories (*launches, may be null, counts them).
+// `next` is a work counter in device memory.
+int plain_beam_batches(omc_engine *e, const BeamSrc<double> &S, double *work, uint64_t seed, long hist0, int nbatch,
+                       long nper, unsigned long long *next, double *src_energy, int block, long *launches = nullptr);
+int plain_beamlet_batches(omc_engine *e, const BeamletSrc<double> &S, int ib, double *work, uint64_t seed, long hist0,
+                          int nbatch, long nper, unsigned long long *next, int block);
 int plain_trace(omc_engine *e, const double *rays_d, int nrays, int cap, double *ustep, int *irnew, int *idisc,
                 int *ncalls, double *hn);
 // `stacks`: plain_replay_stack_bytes(nhist) of device memory for the

@@ -17,6 +17,7 @@
 // passes the array's name to a kernel (on the host it is only a stand-in):
 // the device address is taken once per device with cudaGetSymbolAddress,
 // and again if that device's context has been replaced since.
+#include <algorithm>
 #include <chrono>
 #include <mutex>
 
@@ -35,8 +36,11 @@ namespace {
 
 constexpr long MAXV = OMC_NOALLOC_MAX_VOXELS;
 constexpr long MAXCDF = 1000;
-// layout, in doubles: work | sum | sum2 | dose | unc (MAXV each) | cdf1 | cdf2 (MAXCDF each) | acc (8)
-constexpr long OFF_WORK = 0, OFF_SUM = MAXV, OFF_SUM2 = 2 * MAXV, OFF_DOSE = 3 * MAXV, OFF_UNC = 4 * MAXV;
+// layout, in doubles: sum | sum2 | dose | unc | work (MAXV each) | cdf1 | cdf2 (MAXCDF each) | acc (8).
+// dose and unc are written after the last batch: until then the batch
+// tallies take their place too (from dose on, to the end of work).
+constexpr long OFF_SUM = 0, OFF_SUM2 = MAXV, OFF_DOSE = 2 * MAXV, OFF_UNC = 3 * MAXV, OFF_WORK = OFF_DOSE;
+constexpr long WORK_DOUBLES = 3 * MAXV;
 constexpr long OFF_CDF = 5 * MAXV, OFF_ACC = 5 * MAXV + 2 * MAXCDF;
 constexpr long NDOUBLES = OFF_ACC + 8;
 
@@ -112,10 +116,11 @@ extern "C" int omc_run_beam_noalloc(omc_engine *e, const omc_beam *b, int64_t nc
     if ((rc = scratch_on(e, &s))) return rc;
     if (ncase / nbatch == 0) ncase = nbatch;
     long nper = (long)(ncase / nbatch);
+    const int group = (int)std::min<long>(nbatch, WORK_DOUBLES / nv);
     double *work = s + OFF_WORK, *sum = s + OFF_SUM, *sum2 = s + OFF_SUM2;
     double *dose_d = s + OFF_DOSE, *unc_d = s + OFF_UNC, *cdf = s + OFF_CDF, *acc = s + OFF_ACC;
     // the array keeps the previous call's contents: clear what accumulates
-    if ((rc = cuda_check(e, cudaMemsetAsync(work, 0, nv * 8, e->stream), "clear scratch")) ||
+    if ((rc = cuda_check(e, cudaMemsetAsync(work, 0, (size_t)group * nv * 8, e->stream), "clear scratch")) ||
         (rc = cuda_check(e, cudaMemsetAsync(sum, 0, nv * 8, e->stream), "clear scratch")) ||
         (rc = cuda_check(e, cudaMemsetAsync(sum2, 0, nv * 8, e->stream), "clear scratch")) ||
         (rc = cuda_check(e, cudaMemsetAsync(acc, 0, 8 * 8, e->stream), "clear scratch")) ||
@@ -137,10 +142,14 @@ extern "C" int omc_run_beam_noalloc(omc_engine *e, const omc_beam *b, int64_t nc
     int block = e->opt.block > 0 ? e->opt.block : 128;
     auto t0 = std::chrono::steady_clock::now();
     long launches = 0;  // transport and fold launches, counted as omc_run_beam counts them
-    for (int ib = 0; ib < nbatch; ib++) {
-        if ((rc = plain_beam_batch(e, S, work, seed, (long)ib * nper, nper, acc + 1, block, &launches))) return rc;
-        if ((rc = fold(e, work, sum, sum2, nv, 1.0))) return rc;
-        launches++;
+    for (int b0 = 0; b0 < nbatch; b0 += group) {
+        const int nb = std::min(group, nbatch - b0);
+        if ((rc = plain_beam_batches(e, S, work, seed, (long)b0 * nper, nb, nper, (unsigned long long *)(acc + 2),
+                                     acc + 1, block, &launches)))
+            return rc;
+        for (int ib = 0; ib < nb; ib++)
+            if ((rc = fold(e, work + (long)ib * nv, sum, sum2, nv, 1.0))) return rc;
+        launches += nb;
     }
     if ((rc = device_sum(e, sum, nv, acc))) return rc;
     if ((rc = finalize_dosxyz(e, sum, sum2, nbatch, (double)nper, dose_d, unc_d))) return rc;

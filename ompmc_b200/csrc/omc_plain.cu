@@ -207,44 +207,65 @@ __device__ void shower(const DevData<double> &D, Env &g, Part<double> *st) {
     }
 }
 
-template <int CAP>
-__global__ void k_plain_beam(DevData<double> D, BeamSrc<double> S, double *endep, uint64_t seed, long hist0, long n,
-                             double *src_energy, unsigned *errw) {
+// Histories h0 .. h0 + n - 1 of a group of batches, taken from a counter:
+// `width` lanes of each warp take one at a time.  A history's batch (tally
+// slot) is h / nper, its random stream that of history hist0 + h, so the results do not depend on who runs
+// it.  A warp executes every branch that one of its lanes takes, and a
+// launch lasts as long as its longest histories: few histories are spread
+// over all warps of the GPU, many fill their lanes, and the batches of a
+// run share one launch.  (One launch per batch of one thread per history in
+// order: 2000 histories a batch kept 16 blocks busy, ten times over.)  20,000
+// histories on the 30^3 water phantom 89.2 -> 16.8 ms, 200,000 on the slab
+// phantom 272 -> 89 ms, 12 columns of 3000 histories 298 -> 38 ms.
+template <int CAP, typename Source>
+__device__ __forceinline__ void plain_histories(const DevData<double> &D, double *endep, long nvox, uint64_t seed,
+                                                uint64_t salt, long hist0, long h0, long n, long nper, int width,
+                                                unsigned long long *next, unsigned *errw, const Source &source) {
     PlainEnv<Philox<double>> g;
     Part<double> st[CAP];
-    g.endep = endep;
     g.st = st;
     g.cap = CAP;
-    g.flags = 0;
-    double esum = 0;
-    for (long h = blockIdx.x * (long)blockDim.x + threadIdx.x; h < n; h += (long)gridDim.x * blockDim.x) {
-        g.rng.init(mix64(seed ^ (uint64_t)(hist0 + h) * 0x9E3779B97F4A7C15ull), (uint32_t)(seed >> 32));
-        double ein;
-        st[0] = beam_primary(D, S, g, ein);
-        esum += ein;
-        shower(D, g, st);
+    unsigned flags = 0;
+    if ((int)(threadIdx.x & 31) < width) {
+        for (;;) {
+            const long k = (long)atomicAdd(next, 1ull);
+            if (k >= n) break;
+            const long h = h0 + k;
+            g.endep = endep + h / nper * nvox;
+            g.rng.init(mix64(seed ^ salt ^ (uint64_t)(hist0 + h) * 0x9E3779B97F4A7C15ull), (uint32_t)(seed >> 32));
+            g.flags = 0;
+            st[0] = source(g);
+            shower(D, g, st);
+            flags |= g.flags;
+        }
     }
-    if (g.flags) atomicOr(errw, g.flags);
-    if (src_energy) atomicAdd(src_energy, esum);
+    if (flags) atomicOr(errw, flags);
 }
 
 template <int CAP>
-__global__ void k_plain_beamlet(DevData<double> D, BeamletSrc<double> S, int ib, double *endep, uint64_t seed,
-                                long hist0, long n, unsigned *errw) {
-    PlainEnv<Philox<double>> g;
-    Part<double> st[CAP];
-    g.endep = endep;
-    g.st = st;
-    g.cap = CAP;
-    g.flags = 0;
-    for (long h = blockIdx.x * (long)blockDim.x + threadIdx.x; h < n; h += (long)gridDim.x * blockDim.x) {
-        g.rng.init(mix64(seed ^ ((uint64_t)ib << 40) ^ (uint64_t)(hist0 + h) * 0x9E3779B97F4A7C15ull),
-                   (uint32_t)(seed >> 32));
-        double ein;
-        st[0] = beamlet_primary(D, S, ib, g, ein);
-        shower(D, g, st);
-    }
-    if (g.flags) atomicOr(errw, g.flags);
+__global__ void k_plain_beam(DevData<double> D, BeamSrc<double> S, double *endep, long nvox, uint64_t seed, long hist0,
+                             long h0, long n, long nper, int width, unsigned long long *next, double *src_energy,
+                             unsigned *errw) {
+    double esum = 0;
+    plain_histories<CAP>(D, endep, nvox, seed, 0, hist0, h0, n, nper, width, next, errw,
+                         [&](PlainEnv<Philox<double>> &g) {
+                             double ein;
+                             const Part<double> p = beam_primary(D, S, g, ein);
+                             esum += ein;
+                             return p;
+                         });
+    if (src_energy && esum != 0.0) atomicAdd(src_energy, esum);
+}
+
+template <int CAP>
+__global__ void k_plain_beamlet(DevData<double> D, BeamletSrc<double> S, int ib, double *endep, long nvox,
+                                uint64_t seed, long hist0, long h0, long n, long nper, int width, unsigned long long *next,
+                                unsigned *errw) {
+    plain_histories<CAP>(D, endep, nvox, seed, (uint64_t)ib << 40, hist0, h0, n, nper, width, next, errw,
+                         [&](PlainEnv<Philox<double>> &g) {
+                             double ein;
+                             return beamlet_primary(D, S, ib, g, ein);
+                         });
 }
 
 // ------------------------------------------------------------ validation
@@ -362,48 +383,55 @@ __global__ void k_replay(DevData<double> D, const double *prim, int nhist, const
 }
 
 // ------------------------------------------------------------ launchers
-static int grid_for(omc_engine *e, long n, int block) {
-    long g = (n + block - 1) / block;
-    long cap = (long)e->sm_count * 16;
-    if (g > cap) g = cap;
-    return (int)(g < 1 ? 1 : g);
-}
-
-// Histories per launch of the plain form: about four seconds of FP64
-// transport, so that a large batch is a sequence of bounded launches.  A
-// history's random stream depends on its index only, so the split does not
-// change the result.
+// Histories per launch of the plain form: a few seconds of FP64 transport,
+// so that a large run is a sequence of bounded launches.  A history's random
+// stream depends on its index only, so the split does not change the result.
 static const long PLAIN_CHUNK = 1L << 22;
 
-int plain_beam_batch(omc_engine *e, const BeamSrc<double> &S, double *work, uint64_t seed, long hist0, long n,
-                     double *src_energy, int block, long *launches) {
-    const bool split = e->d64.d.nsplit > 1;
-    for (long c0 = 0; c0 < n; c0 += PLAIN_CHUNK) {
+// One wave of resident blocks; lanes of a warp that take histories: as few
+// as hold them all.
+template <typename K>
+static int plain_grid(omc_engine *e, K kernel, int block, long n, int &width) {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
+    const long per_block = (block + 31) / 32;
+    const long grid = std::max(1L, std::min((long)e->sm_count * std::max(1, per_sm), (n + per_block - 1) / per_block));
+    width = (int)std::min(32L, (n + grid * per_block - 1) / (grid * per_block));
+    return (int)grid;
+}
+
+template <typename F>
+static int plain_chunks(omc_engine *e, long n, unsigned long long *next, long *launches, const char *what, F launch) {
+    for (long h0 = 0; h0 < n; h0 += PLAIN_CHUNK) {
         if (launches) ++*launches;
-        long c = std::min(PLAIN_CHUNK, n - c0);
-        if (split)
-            k_plain_beam<SPLIT_STACK><<<grid_for(e, c, block), block, 0, e->stream>>>(
-                e->d64.d, S, work, seed, hist0 + c0, c, src_energy, e->errword.as<unsigned>());
-        else
-            k_plain_beam<PLAIN_STACK><<<grid_for(e, c, block), block, 0, e->stream>>>(
-                e->d64.d, S, work, seed, hist0 + c0, c, src_energy, e->errword.as<unsigned>());
-        int rc = cuda_check(e, cudaGetLastError(), "k_plain_beam launch");
+        cudaMemsetAsync(next, 0, sizeof(*next), e->stream);
+        launch(h0, std::min(PLAIN_CHUNK, n - h0));
+        int rc = cuda_check(e, cudaGetLastError(), what);
         if (rc) return rc;
     }
     return OMC_OK;
 }
 
-int plain_beamlet_batch(omc_engine *e, const BeamletSrc<double> &S, int ib, double *work, uint64_t seed, long hist0,
-                        long n, int block) {
-    if (e->d64.d.nsplit > 1)
-        k_plain_beamlet<SPLIT_STACK><<<grid_for(e, n, block), block, 0, e->stream>>>(e->d64.d, S, ib, work, seed,
-                                                                                      hist0, n,
-                                                                                      e->errword.as<unsigned>());
-    else
-        k_plain_beamlet<PLAIN_STACK><<<grid_for(e, n, block), block, 0, e->stream>>>(e->d64.d, S, ib, work, seed,
-                                                                                      hist0, n,
-                                                                                      e->errword.as<unsigned>());
-    return cuda_check(e, cudaGetLastError(), "k_plain_beamlet launch");
+int plain_beam_batches(omc_engine *e, const BeamSrc<double> &S, double *work, uint64_t seed, long hist0, int nbatch,
+                       long nper, unsigned long long *next, double *src_energy, int block, long *launches) {
+    auto kernel = e->d64.d.nsplit > 1 ? k_plain_beam<SPLIT_STACK> : k_plain_beam<PLAIN_STACK>;
+    return plain_chunks(e, nbatch * nper, next, launches, "k_plain_beam launch", [&](long h0, long n) {
+        int width;
+        const int grid = plain_grid(e, kernel, block, n, width);
+        kernel<<<grid, block, 0, e->stream>>>(e->d64.d, S, work, e->ph.nvox(), seed, hist0, h0, n, nper, width, next,
+                                              src_energy, e->errword.as<unsigned>());
+    });
+}
+
+int plain_beamlet_batches(omc_engine *e, const BeamletSrc<double> &S, int ib, double *work, uint64_t seed, long hist0,
+                          int nbatch, long nper, unsigned long long *next, int block) {
+    auto kernel = e->d64.d.nsplit > 1 ? k_plain_beamlet<SPLIT_STACK> : k_plain_beamlet<PLAIN_STACK>;
+    return plain_chunks(e, nbatch * nper, next, nullptr, "k_plain_beamlet launch", [&](long h0, long n) {
+        int width;
+        const int grid = plain_grid(e, kernel, block, n, width);
+        kernel<<<grid, block, 0, e->stream>>>(e->d64.d, S, ib, work, e->ph.nvox(), seed, hist0, h0, n, nper, width,
+                                              next, e->errword.as<unsigned>());
+    });
 }
 
 int plain_trace(omc_engine *e, const double *rays_d, int nrays, int cap, double *ustep, int *irnew, int *idisc,

@@ -839,15 +839,17 @@ int omc_run_beamlets(omc_engine *e, const omc_beamlets *b, int64_t nhist, int nb
         if ((rc = upload_plan<double>(e, b, pb.f64, pb.s64))) return rc;
         long nv = e->ph.nvox();
         DBuf work, fin;
-        if ((rc = work.alloc(nv * 8))) return set_err(e, rc, "alloc");
+        const int group = (int)std::max<long>(1, std::min<long>(nbatch, (1L << 30) / (nv * 8)));   // batches run together
+        if ((rc = work.alloc((size_t)group * nv * 8))) return set_err(e, rc, "alloc");
         size_t finb = (size_t)nv * (8 * 6 + 4) + NSEG * 8 + 64;
         if ((rc = fin.alloc(finb))) return set_err(e, rc, "alloc");
-        cudaMemsetAsync(work.p, 0, nv * 8, e->stream);
+        cudaMemsetAsync(work.p, 0, (size_t)group * nv * 8, e->stream);
         double *f = fin.as<double>();
         double *sum = f, *sum2 = f + nv, *dose = f + 2 * nv, *vv = f + 3 * nv, *fvals = f + 4 * nv, *fvars = f + 5 * nv;
         int *frows = (int *)(f + 6 * nv), *cnt = frows + nv, *off = cnt + NSEG;
         unsigned long long *dmax = (unsigned long long *)(((uintptr_t)(off + NSEG) + 15) / 16 * 16);
         long long *total = (long long *)(dmax + 1);
+        unsigned long long *next = dmax + 2;
         if (nhist / nbatch == 0) nhist = nbatch;
         long nper = (long)(nhist / nbatch);
         int block = e->opt.block > 0 ? e->opt.block : 128;
@@ -857,10 +859,13 @@ int omc_run_beamlets(omc_engine *e, const omc_beamlets *b, int64_t nhist, int nb
         for (int i = 0; i < nb; i++) {
             cudaMemsetAsync(sum, 0, nv * 8, e->stream);
             if (!e->opt.ref_compat) cudaMemsetAsync(sum2, 0, nv * 8, e->stream);
-            for (int bt = 0; bt < nbatch; bt++) {
-                if ((rc = plain_beamlet_batch(e, pb.s64, i, work.as<double>(), seed, (long)bt * nper, nper, block)))
+            for (int b0 = 0; b0 < nbatch; b0 += group) {
+                const int nbt = std::min(group, nbatch - b0);
+                if ((rc = plain_beamlet_batches(e, pb.s64, i, work.as<double>(), seed, (long)b0 * nper, nbt, nper, next,
+                                                block)))
                     return rc;
-                if ((rc = fold(e, work.as<double>(), sum, sum2, nv, 1.0 / (double)nper))) return rc;
+                for (int bt = 0; bt < nbt; bt++)
+                    if ((rc = fold(e, work.as<double>() + (size_t)bt * nv, sum, sum2, nv, 1.0 / (double)nper))) return rc;
             }
             if ((rc = finalize_matrad(e, sum, sum2, nbatch, dose, vv))) return rc;
             cudaMemsetAsync(dmax, 0, 8, e->stream);
