@@ -75,44 +75,76 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // 136.5 -> 105.1 ms, code of the kernel 78 -> 63 KB; a fill to 12 at the top
 // of a step and 10 a pass beat 3 / 10 (111.8), 8 / 8 (108.4), 3 / 13 (108.6).
 constexpr int RING = 16;        // numbers a thread holds: ensure() takes up to RING - 3
-__shared__ float s_ring[RING * EV_MAX_BLOCK];
-__device__ __noinline__ void ring_fill(uint32_t block, uint32_t seedw, uint32_t k0, uint32_t k1) {
-    const U4 b = philox4x32_10(U4{block, seedw, 0x6f6d6321u, 0u}, k0, k1);
-    float *c = s_ring + (block & (RING / 4 - 1)) * 4 * EV_MAX_BLOCK + threadIdx.x;
-    c[0] = u01f(b.x);
-    c[EV_MAX_BLOCK] = u01f(b.y);
-    c[2 * EV_MAX_BLOCK] = u01f(b.z);
-    c[3 * EV_MAX_BLOCK] = u01f(b.w);
+// COLS: threads of the block.
+template <int COLS>
+struct RingStore {
+    float v[RING][COLS];
+    uint32_t k0[COLS], k1[COLS];
+};
+template <int COLS>
+__device__ __forceinline__ RingStore<COLS> &ring() {
+    __shared__ RingStore<COLS> r;
+    return r;
 }
+template <int COLS>
+__device__ __noinline__ void ring_fill(uint32_t block, uint32_t seedw) {
+    RingStore<COLS> &r = ring<COLS>();
+    const int t = threadIdx.x;
+    const U4 b = philox4x32_10(U4{block, seedw, 0x6f6d6321u, 0u}, r.k0[t], r.k1[t]);
+    const int row = (block & (RING / 4 - 1)) * 4;
+    r.v[row][t] = u01f(b.x);
+    r.v[row + 1][t] = u01f(b.y);
+    r.v[row + 2][t] = u01f(b.z);
+    r.v[row + 3][t] = u01f(b.w);
+}
+template <int COLS>
 struct RingStream {
-    uint32_t k0, k1, seedw, pos, filled;
+    uint32_t seedw, pos, filled;
     __device__ __forceinline__ void init(uint64_t key, uint32_t seed_word, uint32_t position = 0) {
-        k0 = (uint32_t)key;
-        k1 = (uint32_t)(key >> 32);
+        ring<COLS>().k0[threadIdx.x] = (uint32_t)key;
+        ring<COLS>().k1[threadIdx.x] = (uint32_t)(key >> 32);
         seedw = seed_word;
         pos = position;
         filled = position & ~3u;
     }
     __device__ __forceinline__ uint32_t position() const { return pos; }
+    __device__ __forceinline__ uint64_t key() const {
+        return ((uint64_t)ring<COLS>().k1[threadIdx.x] << 32) | ring<COLS>().k0[threadIdx.x];
+    }
     __device__ __forceinline__ void ensure(int n) {
         while ((int)(filled - pos) < n) {
-            ring_fill(filled >> 2, seedw, k0, k1);
+            ring_fill<COLS>(filled >> 2, seedw);
             filled += 4;
         }
     }
+    // continue at a later position (numbers drawn elsewhere)
+    __device__ __forceinline__ void seek(uint32_t p) {
+        pos = p;
+        if ((int)(filled - p) < 0) filled = p & ~3u;
+    }
     // the caller has asked for it (ensure)
     __device__ __forceinline__ float uni() {
-        const float v = s_ring[(pos & (RING - 1)) * EV_MAX_BLOCK + threadIdx.x];
+        const float v = ring<COLS>().v[pos & (RING - 1)][threadIdx.x];
         pos++;
         return v;
     }
 };
+template <typename Rng>
+struct IsRing {
+    static constexpr bool value = false;
+};
+template <int COLS>
+struct IsRing<RingStream<COLS>> {
+    static constexpr bool value = true;
+};
 
-template <int MAXOUT, typename R = float, typename Rng = Philox<R>>
+template <int MAXOUT, typename R = float, typename Rng = Philox<R>, bool STATS = true>
 struct EvEnv {
-    static constexpr bool kBuffered = std::is_same<Rng, RingStream>::value;
+    static constexpr bool kBuffered = IsRing<Rng>::value;
     Rng rng;
-    double *tally;
+    double *tally;   // the tallies of all slots, nvox apart
+    long nvox;
+    int slot;        // the particle's
     int pend_ir;
     double pend_e;
     Part<R> out[MAXOUT];
@@ -125,7 +157,7 @@ struct EvEnv {
     __device__ R uni() { return rng.uni(); }
     // Consecutive deposits into one voxel are summed before the atomic.
     __device__ void deposit(int ir, R e) {
-        ndep++;
+        if (STATS) ndep++;
         if (ir != pend_ir) {
             flush();
             pend_ir = ir;
@@ -138,7 +170,7 @@ struct EvEnv {
             // tally element (same voxel and tally slot) add once: the
             // group's sum, by its lowest lane (+4-5 % on the served beamlet
             // load and the slab beam over one atomic per lane)
-            double *dst = &tally[pend_ir - 1];
+            double *dst = tally + ((long)slot * nvox + (pend_ir - 1));
             const unsigned act = __activemask();
             const unsigned grp = __match_any_sync(act, (unsigned long long)dst);
             const int lane = threadIdx.x & 31;
@@ -149,13 +181,15 @@ struct EvEnv {
             }
             if (lane == __ffs(grp) - 1) {
                 atomicAdd(dst, tot);
-                natom++;
+                if (STATS) natom++;
             }
         }
         pend_e = 0.0;
         pend_ir = -1;
     }
-    __device__ void cross() { ncross++; }
+    __device__ void cross() {
+        if (STATS) ncross++;
+    }
     __device__ bool tstep_take() { return tleft-- > 0; }
     __device__ bool push(const Part<R> &q) { return push_at(q, rng.position()); }
     // A push made at stream position `pos` (an event run out of line).
@@ -175,7 +209,8 @@ struct EvEnv {
         return true;
     }
     __device__ void err(unsigned f) { flags |= f; }
-    __device__ bool tick() { return ++work < EV_BUDGET; }
+    // (the electron step bounds its own iterations far below the budget)
+    __device__ bool tick() { return kBuffered && !STATS ? true : ++work < EV_BUDGET; }
 };
 
 // A photon event through the out-of-line photon_event_outline: its results
@@ -203,12 +238,18 @@ struct SrcEnv {
 // A queued particle is read once and written once per event, so its loads
 // and stores bypass L1 and are marked streaming (evict first) in L2, which
 // keeps the caches for the tables, the tallies and the kernels' local frames.
+// SHARED: an entry that another block of the same launch wrote (read in L2).
+template <bool SHARED, typename T>
+__device__ __forceinline__ T qread(const T *p) {
+    return SHARED ? __ldcg(p) : __ldcs(p);
+}
+template <bool SHARED = false>
 __device__ __forceinline__ void qload(const Queue &q, int i, Part<float> &p, int &tag, uint32_t &k0, uint32_t &k1,
                                       uint32_t &ctr) {
-    const float4 a = __ldcs(&q.pos[i]);
-    const float4 b = __ldcs(&q.dir[i]);
-    const uint4 c = __ldcs(&q.id[i]);
-    ctr = __ldcs(&q.ctr[i]);
+    const float4 a = qread<SHARED>(&q.pos[i]);
+    const float4 b = qread<SHARED>(&q.dir[i]);
+    const uint4 c = qread<SHARED>(&q.id[i]);
+    ctr = qread<SHARED>(&q.ctr[i]);
     p.x = a.x; p.y = a.y; p.z = a.z; p.u = a.w;
     p.v = b.x; p.w = b.y; p.e = b.z; p.wt = b.w;
     p.ir = (int)c.x;
@@ -217,12 +258,14 @@ __device__ __forceinline__ void qload(const Queue &q, int i, Part<float> &p, int
     k0 = c.z; k1 = c.w;
 }
 
+template <bool SHARED = false>
 __device__ __forceinline__ void qload(const QueueT<double> &q, int i, Part<double> &p, int &tag, uint32_t &k0,
                                       uint32_t &k1, uint32_t &ctr) {
     const double2 *pa = (const double2 *)&q.pos[i], *pb = (const double2 *)&q.dir[i];
-    const double2 a0 = __ldcs(pa), a1 = __ldcs(pa + 1), b0 = __ldcs(pb), b1 = __ldcs(pb + 1);
-    const uint4 c = __ldcs(&q.id[i]);
-    ctr = __ldcs(&q.ctr[i]);
+    const double2 a0 = qread<SHARED>(pa), a1 = qread<SHARED>(pa + 1), b0 = qread<SHARED>(pb),
+                  b1 = qread<SHARED>(pb + 1);
+    const uint4 c = qread<SHARED>(&q.id[i]);
+    ctr = qread<SHARED>(&q.ctr[i]);
     p.x = a0.x; p.y = a0.y; p.z = a1.x; p.u = a1.y;
     p.v = b0.x; p.w = b0.y; p.e = b1.x; p.wt = b1.y;
     p.ir = (int)c.x;
@@ -311,9 +354,9 @@ __device__ __forceinline__ int queue_index(const Q &q, int f) {
 // entry test of electron_step, which the drain applies to the same
 // particle), so that deposit is made here.  It draws no random number, so
 // trajectories do not change.  Returns the particles this lane queued.
-template <int MAXOUT, bool DEFER = false, typename R = float, typename Rng = Philox<R>>
+template <int MAXOUT, bool DEFER = false, typename R = float, typename Env>
 __device__ __forceinline__ int emit(const DevData<R> &D, const QueueT<R> &outP, const QueueT<R> &outE, bool alive,
-                                    const Part<R> &p, EvEnv<MAXOUT, R, Rng> &g, int slot, uint32_t k0, uint32_t k1,
+                                    const Part<R> &p, Env &g, int slot, uint32_t k0, uint32_t k1,
                                     float esplit, int sp = -1, float sr = 0.f, const QueueT<R> *outI = nullptr,
                                     bool defer = false) {
     const unsigned full = 0xffffffffu;
@@ -458,27 +501,24 @@ __device__ __forceinline__ bool split_event(const DevData<R> &D, Env &g, Part<R>
 // D.defer_interact).  `qi`: the interaction queue (EV_ELECTRON with
 // D.defer_interact appends there).
 enum { EV_PHOTON = 0, EV_ELECTRON = 1, EV_SPLIT = 2, EV_INTERACT = 3, EV_ELECTRON_DEFER = 4 };
-template <int KIND, typename R = float>
+template <int KIND, typename R = float, bool STATS = true>
 __device__ __forceinline__ void transport_events(const DevData<R> &D, const QueueT<R> &in, const QueueT<R> &outP,
                                                  const QueueT<R> &outE, double *tallies, long nvox, Ctl *ctl,
                                                  uint32_t seedw, ServeDev *sd, int nbmax, const QueueT<R> &qi) {
     constexpr int MAXOUT = KIND == EV_SPLIT ? EV_MAXOUT_SPLIT : EV_MAXOUT;
     const unsigned full = 0xffffffffu;
     constexpr bool ELECTRON = KIND == EV_ELECTRON || KIND == EV_ELECTRON_DEFER;
-    using Rng = typename std::conditional<KIND == EV_ELECTRON_DEFER && sizeof(R) == 4, RingStream, Philox<R>>::type;
-    using Env = EvEnv<MAXOUT, R, Rng>;
+    using Rng = typename std::conditional<KIND == EV_ELECTRON_DEFER && sizeof(R) == 4, RingStream<EV_MAX_BLOCK>, Philox<R>>::type;
+    using Env = EvEnv<MAXOUT, R, Rng, STATS>;
     const int kq = ELECTRON ? 1 : (KIND == EV_INTERACT ? 2 : 0);
     const int ks = KIND == EV_PHOTON || KIND == EV_SPLIT ? 0 : 1;   // counters: photon or electron
-    const int n = queue_size(in);
-    const int tsteps = ctl->tsteps;
-    const float esplit = ctl->esplit;
     const int lane = threadIdx.x & 31;
-    unsigned flags = 0;
     unsigned c_ev = 0, c_steps = 0, c_cross = 0, c_dep = 0, c_atom = 0;
     for (int guard = 0; guard < (1 << 26); guard++) {
         int base = 0;
         if (lane == 0) base = atomicAdd(&ctl->fetch[kq], 32);
         base = __shfl_sync(full, base, 0);
+        const int n = queue_size(in);
         if (base >= n) break;
         const bool valid = base + lane < n;
         const int i = valid ? queue_index(in, base + lane) : 0;
@@ -495,13 +535,15 @@ __device__ __forceinline__ void transport_events(const DevData<R> &D, const Queu
         const int slot = tag >> 2;
         Env g;
         g.rng.init(((uint64_t)k1 << 32) | k0, seedw, pos);
-        g.tally = tallies + (long)slot * nvox;
+        g.tally = tallies;
+        g.nvox = nvox;
+        g.slot = slot;
         g.pend_ir = -1;
         g.pend_e = 0.0;
         g.nout = 0;
         g.flags = 0;
         g.work = 0;
-        g.tleft = tsteps;
+        g.tleft = ctl->tsteps;
         g.ncross = g.ndep = g.natom = 0;
         bool alive = false, defer = false;
         if (valid) {
@@ -519,18 +561,26 @@ __device__ __forceinline__ void transport_events(const DevData<R> &D, const Queu
             }
             g.flush();
         }
+        if constexpr (Env::kBuffered) {
+            const uint64_t key = g.rng.key();
+            k0 = (uint32_t)key;
+            k1 = (uint32_t)(key >> 32);
+        }
+        const float esplit = ctl->esplit;
         int emitted = KIND == EV_ELECTRON_DEFER
-                          ? emit<MAXOUT, true, R, Rng>(D, outP, outE, alive, p, g, slot, k0, k1, esplit, sp, sr, &qi, defer)
-                          : emit<MAXOUT, false, R, Rng>(D, outP, outE, alive, p, g, slot, k0, k1, esplit, sp, sr);
+                          ? emit<MAXOUT, true, R>(D, outP, outE, alive, p, g, slot, k0, k1, esplit, sp, sr, &qi, defer)
+                          : emit<MAXOUT, false, R>(D, outP, outE, alive, p, g, slot, k0, k1, esplit, sp, sr);
         if (sd) add_live(sd->live, nbmax, valid ? slot : 0, valid ? emitted - 1 : 0, full);
-        flags |= g.flags;
-        c_ev += valid;
-        c_steps += g.work;
-        c_cross += g.ncross;
-        c_dep += g.ndep;
-        c_atom += g.natom;
+        report_flags(ctl, g.flags, full);
+        if (STATS) {
+            c_ev += valid;
+            c_steps += g.work;
+            c_cross += g.ncross;
+            c_dep += g.ndep;
+            c_atom += g.natom;
+        }
     }
-    report_flags(ctl, flags, full);
+    if (!STATS) return;
     if (KIND != EV_INTERACT) report_count(&ctl->st_events[ks], c_ev, full);
     report_count(&ctl->st_steps[ks], c_steps, full);
     report_count(&ctl->st_cross[ks], c_cross, full);
@@ -558,11 +608,11 @@ __global__ void __launch_bounds__(EV_MAX_BLOCK) k_photon_split_step(DevData<floa
 // cycle's budget of tstep-loop iterations each, then the particle is
 // re-queued.  The step is latency bound; the occupancy it is compiled for
 // (electron_minb) trades resident warps against spilled local frames.
-template <bool DEFER, typename R = float>
+template <bool DEFER, typename R = float, bool STATS = true>
 __global__ void __launch_bounds__(EV_MAX_BLOCK, electron_minb<R>())
     k_electron_step(DevData<R> D, QueueT<R> in, QueueT<R> outP, QueueT<R> outE, double *tallies, long nvox, Ctl *ctl,
                     uint32_t seedw, ServeDev *sd, int nbmax, QueueT<R> qi) {
-    transport_events<DEFER ? EV_ELECTRON_DEFER : EV_ELECTRON, R>(D, in, outP, outE, tallies, nvox, ctl, seedw, sd,
+    transport_events<DEFER ? EV_ELECTRON_DEFER : EV_ELECTRON, R, STATS>(D, in, outP, outE, tallies, nvox, ctl, seedw, sd,
                                                                   nbmax, qi);
 }
 
@@ -570,7 +620,8 @@ __global__ void __launch_bounds__(EV_MAX_BLOCK, electron_minb<R>())
 // (D.defer_interact) or in place.
 template <typename R = float>
 static TransportKernelT<R> electron_kernel(const omc_engine *e) {
-    return e->d32.d.defer_interact ? k_electron_step<true, R> : k_electron_step<false, R>;
+    if (!e->d32.d.defer_interact) return k_electron_step<false, R>;
+    return e->opt.profile ? k_electron_step<true, R> : k_electron_step<true, R, false>;
 }
 
 // Discrete interactions of the electrons the electron kernel left at their
@@ -587,22 +638,50 @@ __global__ void __launch_bounds__(EV_MAX_BLOCK) k_electron_interact(DevData<R> D
 // Once every history is injected and few particles remain, transport
 // cycles launch mostly idle kernels whose duration is the latency of their
 // longest events, and each particle waits a whole cycle between events.
-// The drain runs each remaining particle to the end of its sub-history in
-// one launch instead: one thread per queued particle, its secondaries on a
-// local stack.  Every particle keeps its own random stream and its
-// secondaries get the keys emit() gives them, electrons run to their
-// interaction without a budget (budgets do not change trajectories) and
-// interactions are sampled in place (the same draws as the interaction
-// kernel), so the dose is the one the cycles would have produced, up to
-// the summation order of the FP64 tallies.  SPLIT: photons are split rays
-// (nsplit > 1) whose state (next sub-photon, survivor, offset) rides on the
-// stack with them, as in the photon queues.
+// The drain runs the remaining particles to the end of their sub-histories
+// in one launch instead.  Every particle keeps its own random stream and its
+// secondaries get the keys emit() gives them, and interactions are sampled
+// in place (the same draws as the interaction kernel), so the dose is the
+// one the cycles would have produced, up to the summation order of the FP64
+// tallies.
+//
+// A task is a particle with everything it gives rise to; a lane runs one
+// task at a time, its secondaries on a local stack.  Electrons run one
+// tstep-loop iteration at a time (budgets do not change trajectories), so
+// that the lanes of a warp meet again soon.  A lane's electron step costs the
+// instructions of every branch that any lane of its warp takes (a warp of one
+// particle takes 4.3 us a step where nothing else runs), so the particles
+// are spread over all resident warps, and a warp that has run out of work is
+// given another's oldest pending particle, or one that a crowded warp has in
+// hand, through a pool in global memory: the launch ends with the longest
+// track, not with the longest sub-history.
+//
+// The warps of an SM are bound by the instructions they fetch: fifteen
+// warps of one particle each took 50 us an iteration where three took 15
+// and one 11.5 (a miss of the instruction cache is served every 23 cycles
+// or so).  So the one block of an SM runs its iterations, and the
+// transport, interactions and photons of an iteration, in step: its warps
+// share what they fetch.  37 k particles on the slab phantom, ms a launch:
+// one particle a thread in order 20.0; spread, donating, numbers from shared
+// memory 16.5; blocks of 256 in step 16.0; of 512, in step by phase 14.8.
+//
+// The pool needs no lock: a warp without work draws a ticket (drain_head);
+// tickets below the number of queued particles are those, the others wait
+// for the pool entry of their number to be marked ready, or for the end.
+// A lane donates only while tickets outnumber entries (compare and swap), so
+// an entry always has a taker.  The launch is over when as many tasks are
+// done as were made.  Lanes wait only when no particle is left unclaimed, so
+// blocks that are not resident yet hold nobody up, and every wait has a
+// limit.
+// SPLIT: photons are split rays (nsplit > 1) whose state (next sub-photon,
+// survivor, offset) rides along with them, as in the photon queues.
 constexpr int DRAIN_STACK = 48;
-// 4 resident blocks of 128 per SM: up to 128 registers and no spills.  The
-// drain's length is the latency of its longest sub-history in one thread,
-// which spilled registers lengthen; it never needs more lanes than
-// particles (1.2 % faster on slab64 than 8 blocks at 64 registers).
-constexpr int DRAIN_BLOCK = 128;
+// One block of 512 per SM: up to 128 registers, which keep the step's state
+// out of memory.
+constexpr int DRAIN_BLOCK = 512;
+constexpr int DRAIN_TSTEPS = 1;               // tstep-loop iterations a turn
+constexpr int DRAIN_POOL = 1 << 18;           // donations per launch; beyond them lanes keep their work
+constexpr int DRAIN_POLLS = 1 << 24;          // looks of an idle block at the pool (1 us each) before it gives up
 
 template <typename R>
 struct DrainPart {
@@ -612,11 +691,348 @@ struct DrainPart {
     float sr;
 };
 
-// STATS (profiled runs): record the largest sub-history a thread ran.
-template <bool SPLIT, bool STATS = false, typename R = float>
-__global__ void __launch_bounds__(DRAIN_BLOCK, 4) k_drain(DevData<R> D, QueueT<R> qP, QueueT<R> qE, double *tallies,
-                                                        long nvox, Ctl *ctl, uint32_t seedw) {
+__device__ __forceinline__ int ld_volatile(const int *p) { return *(const volatile int *)p; }
+
+// The environment of a sampler run on copies: g's stream, with nothing
+// pending, and back into g with what the sampler did.
+template <typename Env, typename Host>
+__device__ __forceinline__ void sampler_env(Env &h, const Host &g) {
+    h.rng.init(g.rng.key(), g.rng.seedw, g.rng.position());
+    h.tally = g.tally;
+    h.nvox = g.nvox;
+    h.slot = g.slot;
+    h.pend_ir = g.pend_ir;
+    h.pend_e = g.pend_e;
+    h.nout = 0;
+    h.flags = 0;
+    h.work = g.work;
+    h.tleft = 0;
+    h.ncross = h.ndep = h.natom = 0;
+}
+template <int MAXOUT, typename Host, typename Env>
+__device__ __forceinline__ void sampled(Host &g, const Env &h) {
+    if constexpr (Host::kBuffered) g.rng.seek(h.rng.position());
+    else g.rng = h.rng;
+    g.pend_ir = h.pend_ir;
+    g.pend_e = h.pend_e;
+    g.nout = h.nout;
+#pragma unroll
+    for (int k = 0; k < MAXOUT; k++) {
+        g.out[k] = h.out[k];
+        g.out_pos[k] = h.out_pos[k];
+    }
+    g.flags |= h.flags;
+    g.work = h.work;
+    g.ncross += h.ncross;
+    g.ndep += h.ndep;
+    g.natom += h.natom;
+}
+
+// An electron's turn in the drain, out of line and by value, as a photon's
+// is: its registers are then its own, not the drain's (inlined, the served
+// load took 10 % longer).
+template <typename R, typename Rng, bool STATS>
+struct ElectronEventOut {
+    Part<R> p, q;
+    Rng rng;
+    int pend_ir;
+    double pend_e;
+    uint32_t qpos;
+    int r, nq, work, ncross, ndep, natom;
+    unsigned flags;
+};
+template <typename R, typename Rng, bool STATS>
+__device__ __noinline__ ElectronEventOut<R, Rng, STATS> electron_event_outline(const DevData<R> &D, Part<R> p, Rng rng,
+                                                                               double *tally, long nvox, int slot,
+                                                                               int pend_ir, double pend_e) {
+    EvEnv<1, R, Rng, STATS> g;
+    g.rng = rng;
+    g.tally = tally;
+    g.nvox = nvox;
+    g.slot = slot;
+    g.pend_ir = pend_ir;
+    g.pend_e = pend_e;
+    g.nout = 0;
+    g.flags = 0;
+    g.work = 0;
+    g.tleft = DRAIN_TSTEPS;
+    g.ncross = g.ndep = g.natom = 0;
+    ElectronEventOut<R, Rng, STATS> o;
+    o.r = electron_step<R, EvEnv<1, R, Rng, STATS>, true>(D, g, p);
+    o.p = p;
+    o.q = g.out[0];
+    o.qpos = g.out_pos[0];
+    o.nq = g.nout;
+    o.rng = g.rng;
+    o.pend_ir = g.pend_ir;
+    o.pend_e = g.pend_e;
+    o.work = g.work;
+    o.ncross = g.ncross;
+    o.ndep = g.ndep;
+    o.natom = g.natom;
+    o.flags = g.flags;
+    return o;
+}
+
+// STATS (profiled runs): count, and record the largest sub-history a lane ran.
+template <bool SPLIT, bool STATS = false>
+__global__ void __launch_bounds__(DRAIN_BLOCK, 1)
+    k_drain(DevData<float> D, Queue qP, Queue qE, Queue pool, int *ready, double *tallies, long nvox, Ctl *ctl,
+            uint32_t seedw) {
     constexpr int MAXOUT = SPLIT ? EV_MAXOUT_SPLIT : EV_MAXOUT;
+    using R = float;
+    using Rng = RingStream<DRAIN_BLOCK>;
+    using Env = EvEnv<MAXOUT, R, Rng, STATS>;
+    const unsigned full = 0xffffffffu;
+    const int np = queue_size(qP), ne = queue_size(qE);
+    const int n = np + ne;
+    const int pool_cap = min(DRAIN_POOL, pool.cap);
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * (DRAIN_BLOCK / 32);
+    const bool takes = lane < (n + warps - 1) / warps;
+    DrainPart<R> st[DRAIN_STACK];   // the task's pending particles
+    int depth = 0;
+    Part<R> p;                      // the particle in hand
+    p.iq = 0;
+    int sp = -1;
+    float sr = 0.f;
+    bool busy = false, alone = false;
+    int ticket = -1;
+    Env g;
+    g.tally = tallies;
+    g.nvox = nvox;
+    unsigned c_ev[2] = {0, 0}, c_steps[2] = {0, 0}, c_cross[2] = {0, 0}, c_dep[2] = {0, 0}, c_atom = 0;
+    int x_ev = 0, x_chain = 0, x_steps = 0;   // this task: events, events of its first particle, steps
+    int first_at = 0;                         // where the first particle is: stack entry, -1 in hand, -2 gone
+    for (int idle = 0;;) {
+        // the warps of a block take their iterations, and the phases of an
+        // iteration, together, so that they share the instructions they fetch
+        const bool block_busy = __syncthreads_or(busy);
+        if (!busy && ticket < 0 && takes && ((lane == 0 && alone) || ld_volatile(&ctl->drain_head) < n))
+            ticket = atomicAdd(&ctl->drain_head, 1);
+        if (!busy && ticket >= 0) {
+            const int k = ticket - n;
+            int tag = 0;
+            uint32_t k0 = 0, k1 = 0, pos = 0;
+            if (k < 0) {
+                const QueueT<R> &q = ticket < np ? qP : qE;
+                const int qi = queue_index(q, ticket < np ? ticket : ticket - np);
+                qload(q, qi, p, tag, k0, k1, pos);
+                sp = (SPLIT && q.sp) ? q.sp[qi] : -1;
+                sr = (SPLIT && q.sr) ? q.sr[qi] : 0.f;
+                busy = true;
+            } else if (k < pool_cap && ld_volatile(&ready[k])) {
+                __threadfence();
+                qload<true>(pool, k, p, tag, k0, k1, pos);
+                sp = SPLIT ? __ldcg(&pool.sp[k]) : -1;
+                sr = SPLIT ? __ldcg(&pool.sr[k]) : 0.f;
+                busy = true;
+            }
+            if (busy) {
+                ticket = -1;
+                g.slot = tag >> 2;
+                g.rng.init(((uint64_t)k1 << 32) | k0, seedw, pos);
+                g.pend_ir = -1;
+                g.pend_e = 0.0;
+                g.flags = 0;
+                g.natom = 0;
+                x_ev = x_chain = x_steps = 0;
+                first_at = -1;
+            }
+        }
+        alone = !__any_sync(full, busy);
+        if (!block_busy) {
+            // nothing in hand in this block: over, or wait for a donation.
+            // Tasks done are read before tasks made: when they agree nobody
+            // is left who could make more.
+            int over = 0;
+            if (threadIdx.x == 0) {
+                over = ld_volatile(&ctl->drain_done) >= n + min(ld_volatile(&ctl->drain_tail), pool_cap);
+                if (over) {
+                    const int done = ld_volatile(&ctl->drain_done);
+                    __threadfence();
+                    over = done >= n + min(ld_volatile(&ctl->drain_tail), pool_cap);
+                }
+            }
+            if (__syncthreads_or(over)) break;
+            if (++idle > DRAIN_POLLS) {
+                if (threadIdx.x == 0) atomicOr(&ctl->flags, (unsigned)ERR_LOOP);
+                break;
+            }
+            if (alone) __nanosleep(1000);
+        } else {
+            idle = 0;
+        }
+        const uint64_t pkey = g.rng.key();
+        g.nout = 0;
+        g.work = 0;
+        g.ncross = g.ndep = 0;
+        const int kind = p.iq == 0 ? 0 : 1;
+        bool alive = false;
+        int r = E_DEAD;
+        if (busy && kind == 1) {
+            const ElectronEventOut<R, Rng, STATS> o = electron_event_outline<R, Rng, STATS>(
+                D, p, g.rng, tallies, nvox, g.slot, g.pend_ir, g.pend_e);
+            r = o.r;
+            p = o.p;
+            g.rng = o.rng;
+            g.pend_ir = o.pend_ir;
+            g.pend_e = o.pend_e;
+            g.flags |= o.flags;
+            g.work = o.work;
+            g.ncross = o.ncross;
+            g.ndep = o.ndep;
+            g.natom += o.natom;
+            if (o.nq) g.push_at(o.q, o.qpos);
+            alive = r != E_DEAD;
+        }
+        __syncthreads();
+        if (r == E_INTERACT) {
+            // the samplers run out of line on copies, so that the lane's
+            // own particle and environment stay in registers
+            EvEnv<MAXOUT, R> h;
+            Part<R> q = p;
+            sampler_env(h, g);
+            electron_interact(D, h, q);
+            p = q;
+            sampled<MAXOUT>(g, h);
+        }
+        __syncthreads();
+        if (!busy) continue;
+        if (kind == 0) {
+            EvEnv<MAXOUT, R> h;
+            sampler_env(h, g);
+            if constexpr (SPLIT) {
+                Part<R> q = p;
+                int hsp = sp;
+                float hsr = sr;
+                alive = split_event(D, h, q, hsp, hsr);
+                sp = hsp;
+                sr = hsr;
+                p = q;
+            } else {
+                alive = photon_event(D, h, p);
+            }
+            sampled<MAXOUT>(g, h);
+        }
+        if (STATS) {
+            c_ev[kind]++;
+            c_steps[kind] += g.work;
+            c_cross[kind] += g.ncross;
+            c_dep[kind] += g.ndep;
+            x_chain += first_at == -1;
+            x_steps += g.work;
+        }
+        x_ev++;
+        if (alive && !(p.e == p.e && p.x == p.x && p.u == p.u)) {
+            g.flags |= ERR_NAN;
+            alive = false;
+        }
+        if (alive && p.iq == 0 && p.wt == R(0)) alive = false;
+        if (!alive && first_at == -1) first_at = -2;
+        // children first: the parent waits on the stack, which then holds
+        // one particle a generation (split rays: a few)
+        for (int k = 0; k < g.nout; k++) {
+            const Part<R> &s2 = g.out[k];
+            if (!(s2.e == s2.e && s2.x == s2.x && s2.u == s2.u)) {
+                g.flags |= ERR_NAN;
+                continue;
+            }
+            if (s2.iq == 0 && s2.wt == R(0)) continue;
+            const uint64_t ck = mix64(pkey * 0x9E3779B97F4A7C15ull + ((uint64_t)g.out_pos[k] << 1) + 1u +
+                                      ((uint64_t)k << 40));
+            if (alive) {
+                if (depth >= DRAIN_STACK) {
+                    g.flags |= ERR_STACK;
+                    continue;
+                }
+                const uint64_t key = g.rng.key();
+                st[depth].p = p;
+                st[depth].k0 = (uint32_t)key;
+                st[depth].k1 = (uint32_t)(key >> 32);
+                st[depth].pos = g.rng.position();
+                st[depth].sp = sp;
+                st[depth].sr = sr;
+                if (first_at == -1) first_at = depth;
+                depth++;
+            }
+            p = s2;
+            g.rng.init(ck, seedw);
+            sp = -1;
+            sr = 0.f;
+            alive = true;
+        }
+        if (x_ev > (1 << 22)) {
+            g.flags |= ERR_LOOP;
+            alive = false;
+            depth = 0;
+        }
+        if (!alive && depth > 0) {
+            depth--;
+            p = st[depth].p;
+            g.rng.init(((uint64_t)st[depth].k1 << 32) | st[depth].k0, seedw, st[depth].pos);
+            sp = st[depth].sp;
+            sr = st[depth].sr;
+            if (first_at == depth) first_at = -1;
+            alive = true;
+        }
+        // warps without work wait for some: the oldest pending particle of a
+        // lane, which has the most of its track left, or, where the warp has
+        // other lanes at work, the particle in hand becomes a task of its own
+        const unsigned working = __activemask();
+        if (depth > 0 || (alive && lane != __ffs(working) - 1)) {
+            const int tail = ld_volatile(&ctl->drain_tail);
+            if (tail < pool_cap && ld_volatile(&ctl->drain_head) > n + tail &&
+                atomicCAS(&ctl->drain_tail, tail, tail + 1) == tail) {
+                if (depth > 0) {
+                    const DrainPart<R> &e = st[0];
+                    qstore(pool, tail, e.p, g.slot, e.k0, e.k1, e.pos, e.sp, e.sr);
+                    depth--;
+                    for (int i = 0; i < depth; i++) st[i] = st[i + 1];
+                    first_at = first_at == 0 ? -2 : (first_at > 0 ? first_at - 1 : first_at);
+                } else {
+                    const uint64_t key = g.rng.key();
+                    qstore(pool, tail, p, g.slot, (uint32_t)key, (uint32_t)(key >> 32), g.rng.position(), sp, sr);
+                    alive = false;
+                }
+                __threadfence();
+                *(volatile int *)&ready[tail] = 1;
+            }
+        }
+        if (!alive) {
+            g.flush();
+            if (STATS) c_atom += g.natom;     // tally atomics of the whole task
+            if (g.flags) atomicOr(&ctl->flags, g.flags);
+            busy = false;
+            if (STATS) {
+                atomicMax(&ctl->drain_max_events, x_ev);
+                atomicMax(&ctl->drain_max_chain, x_chain);
+                atomicMax(&ctl->drain_max_steps, x_steps);
+            }
+            __threadfence();
+            atomicAdd(&ctl->drain_done, 1);
+        }
+    }
+    if (!STATS) return;
+    __syncwarp();
+    for (int k = 0; k < 2; k++) {
+        report_count(&ctl->st_events[k], c_ev[k], full);
+        report_count(&ctl->st_steps[k], c_steps[k], full);
+        report_count(&ctl->st_cross[k], c_cross[k], full);
+        report_count(&ctl->st_dep[k], c_dep[k], full);
+    }
+    report_count(&ctl->st_atom[1], c_atom, full);
+}
+
+// The FP64 event form's drain: one thread per queued particle in order, with
+// its secondaries on the local stack.  FP64 rounding is the compiler's choice
+// kernel by kernel, and the accuracy study's results rest on this one's.
+// STATS (profiled runs): record the largest sub-history a thread ran.
+constexpr int DRAIN64_BLOCK = 128;
+template <bool STATS = false, typename R = double>
+__global__ void __launch_bounds__(DRAIN64_BLOCK, 4) k_drain64(DevData<R> D, QueueT<R> qP, QueueT<R> qE, double *tallies,
+                                                          long nvox, Ctl *ctl, uint32_t seedw) {
+    constexpr int MAXOUT = EV_MAXOUT;
     const int np = queue_size(qP), ne = queue_size(qE);
     const int n = np + ne;
     DrainPart<R> st[DRAIN_STACK];
@@ -628,10 +1044,10 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 4) k_drain(DevData<R> D, QueueT<R
         int tag = 0;
         const int qi = queue_index(q, t < np ? t : t - np);
         qload(q, qi, st[0].p, tag, st[0].k0, st[0].k1, st[0].pos);
-        st[0].sp = (SPLIT && q.sp) ? q.sp[qi] : -1;
-        st[0].sr = (SPLIT && q.sr) ? q.sr[qi] : 0.f;
         EvEnv<MAXOUT, R> g;
-        g.tally = tallies + (long)(tag >> 2) * nvox;
+        g.tally = tallies;
+        g.nvox = nvox;
+        g.slot = tag >> 2;
         g.pend_ir = -1;
         g.pend_e = 0.0;
         g.flags = 0;
@@ -657,11 +1073,8 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 4) k_drain(DevData<R> D, QueueT<R
             g.tleft = 1 << 30;
             g.ncross = g.ndep = 0;
             const int kind = p.iq == 0 ? 0 : 1;
-            int sp = e.sp;
-            float sr = e.sr;
             bool alive;
             if (kind == 1) alive = electron_step<R, EvEnv<MAXOUT, R>, false>(D, g, p) == E_ALIVE;
-            else if constexpr (SPLIT) alive = split_event(D, g, p, sp, sr);
             else alive = photon_event(D, g, p);
             c_ev[kind]++;
             x_steps += g.work;
@@ -676,8 +1089,6 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 4) k_drain(DevData<R> D, QueueT<R
             if (alive) {
                 e.p = p;
                 e.pos = g.rng.position();
-                e.sp = sp;
-                e.sr = sr;
             } else {
                 top--;
                 first_alive = first_alive && !first;
@@ -700,8 +1111,6 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 4) k_drain(DevData<R> D, QueueT<R
                 st[top].k0 = (uint32_t)ck;
                 st[top].k1 = (uint32_t)(ck >> 32);
                 st[top].pos = 0;
-                st[top].sp = -1;
-                st[top].sr = 0.f;
             }
         }
         g.flush();
@@ -885,8 +1294,13 @@ static void size_grids(omc_engine *e, EventStateT<R> &S) {
     int bi = 0, bd = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bi, k_electron_interact<R>, S.block, 0);
     S.grid_i = e->sm_count * std::max(1, bi);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain<false, false, R>, DRAIN_BLOCK, 0);
-    S.drain_lanes = e->sm_count * std::max(1, bd) * DRAIN_BLOCK;
+    if constexpr (sizeof(R) == 4) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain<false, false>, DRAIN_BLOCK, 0);
+        S.drain_lanes = e->sm_count * std::max(1, bd) * DRAIN_BLOCK;
+    } else {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain64<false>, DRAIN64_BLOCK, 0);
+        S.drain_lanes = e->sm_count * std::max(1, bd) * DRAIN64_BLOCK;
+    }
     S.lanes = S.grid_e * S.block;
 }
 
@@ -923,6 +1337,7 @@ static int event_prepare_t(omc_engine *e) {
     S.ctl_d = S.ctl.template as<Ctl>();
     for (int i = 0; i < 4; i++)
         if ((rc = alloc_queue(e, S.buf[i], S.q[i], S.cap, &S.ctl_d->cnt[i], &S.ctl_d->cnt_hi[i]))) return rc;
+    if (sizeof(R) == 4 && (rc = S.drain_ready.alloc(DRAIN_POOL * sizeof(int)))) return set_err(e, rc, "drain pool allocation failed");
     if (e->d32.d.nsplit > 1 && sizeof(R) == 4) {
         // splitting state of the two photon queues (A and B)
         for (int k = 0; k < 2; k++) {
@@ -1071,16 +1486,25 @@ template <typename R = float>
 static void launch_drain(omc_engine *e, int iph, long long left, double *tallies, uint32_t seedw,
                          bool stats = false) {
     EventStateT<R> &S = *state_of<R>(e);
-    long long g = (left + DRAIN_BLOCK - 1) / DRAIN_BLOCK;
-    g = std::max(1LL, std::min(g, (long long)S.drain_lanes / DRAIN_BLOCK * 4));
     const DevData<R> D = event_data<R>(e);
-    void (*kd)(DevData<R>, QueueT<R>, QueueT<R>, double *, long, Ctl *, uint32_t);
-    if constexpr (sizeof(R) == 4)
-        kd = D.nsplit > 1 ? (stats ? k_drain<true, true, R> : k_drain<true, false, R>)
-                          : (stats ? k_drain<false, true, R> : k_drain<false, false, R>);
-    else
-        kd = stats ? k_drain<false, true, R> : k_drain<false, false, R>;
-    kd<<<(int)g, DRAIN_BLOCK, 0, e->stream>>>(D, S.q[iph], S.q[iph + 1], tallies, e->ph.nvox(), S.ctl_d, seedw);
+    if constexpr (sizeof(R) == 8) {
+        const long long g = std::max(1LL, std::min((left + DRAIN64_BLOCK - 1) / DRAIN64_BLOCK,
+                                                   (long long)S.drain_lanes / DRAIN64_BLOCK * 4));
+        auto kd = stats ? k_drain64<true> : k_drain64<false>;
+        kd<<<(int)g, DRAIN64_BLOCK, 0, e->stream>>>(D, S.q[iph], S.q[iph + 1], tallies, e->ph.nvox(), S.ctl_d, seedw);
+    } else {
+        // a warp per particle, up to one wave of resident blocks
+        const long long warps = DRAIN_BLOCK / 32;
+        const long long g = std::max(1LL, std::min((left + warps - 1) / warps, (long long)S.drain_lanes / DRAIN_BLOCK));
+        auto kd = D.nsplit > 1 ? (stats ? k_drain<true, true> : k_drain<true, false>)
+                               : (stats ? k_drain<false, true> : k_drain<false, false>);
+        // the pool: the photon output queue, empty between cycles, and its flags
+        int *ready = S.drain_ready.template as<int>();
+        cudaMemsetAsync(ready, 0, DRAIN_POOL * sizeof(int), e->stream);
+        cudaMemsetAsync(&S.ctl_d->drain_head, 0, 4 * sizeof(int), e->stream);
+        kd<<<(int)g, DRAIN_BLOCK, 0, e->stream>>>(D, S.q[iph], S.q[iph + 1], S.q[iph ^ 2], ready, tallies, e->ph.nvox(),
+                                                  S.ctl_d, seedw);
+    }
 }
 
 // Profiled transport: cycles launched one by one with events around each

@@ -64,6 +64,10 @@ struct Ctl {
     // drain: the largest sub-history one thread ran (events, events of the
     // particle it started from, transport steps)
     int drain_max_events, drain_max_chain, drain_max_steps, drain_pad;
+    // drain: queued particles taken, particles donated to the pool, taken
+    // from it, tasks done (one 16-byte load)
+    alignas(16) int drain_head;
+    int drain_tail, drain_over, drain_done;
 };
 
 // Per-kernel profile of the last run made with options.profile = 1.
@@ -92,6 +96,7 @@ struct EventStateT {
     DBuf int_buf;             // electrons at their discrete interaction (defer_interact)
     QueueT<R> qi;
     QueueT<R> q[4];
+    DBuf drain_ready;         // the drain's pool: entries published
     DBuf ctl;
     Ctl *ctl_d = nullptr;
     int block = 256;

@@ -75,6 +75,23 @@ OMC_HD float m_mul(float a, float b) {
     return a * b;
 #endif
 }
+// Sums of products in the electron step, with the product that is
+// contracted into the sum said explicitly: which one the compiler picks
+// depends on the code around, and every FP32 kernel has to round a
+// trajectory alike.  sum_fma1 and sum_fma2 are a*b + c*d with a*b,
+// respectively c*d, contracted; sum_sq<1> and <2> the same for a*a + b*b
+// (<0>: the compiler's choice).  FP64 is left to the compiler (the plain form
+// contracts nothing).
+OMC_HD double sum_fma1(double a, double b, double c, double d) { return a * b + c * d; }
+OMC_HD float sum_fma1(float a, float b, float c, float d) { return fmaf(a, b, m_mul(c, d)); }
+OMC_HD double sum_fma2(double a, double b, double c, double d) { return a * b + c * d; }
+OMC_HD float sum_fma2(float a, float b, float c, float d) { return fmaf(c, d, m_mul(a, b)); }
+template <int W>
+OMC_HD double sum_sq(double a, double b) { return a * a + b * b; }
+template <int W>
+OMC_HD float sum_sq(float a, float b) {
+    return W == 1 ? fmaf(a, a, m_mul(b, b)) : W == 2 ? fmaf(b, b, m_mul(a, a)) : a * a + b * b;
+}
 template <typename R> OMC_HD R sq(R x) { return x * x; }
 template <typename R> OMC_HD bool m_abs_lt(R a, R b) { return (a < R(0) ? -a : a) < b; }
 
@@ -82,9 +99,11 @@ template <typename R> OMC_HD bool m_abs_lt(R a, R b) { return (a < R(0) ? -a : a
 // rounding drift never accumulates and the trajectory does not depend on
 // where events are cut; the FP64 form is left untouched (its trajectories
 // stay bit-identical to the reference's).
+template <int W = 0>
 OMC_HD void renorm_dir(double &, double &, double &) {}
+template <int W = 0>
 OMC_HD void renorm_dir(float &u, float &v, float &w) {
-    float n2 = u * u + v * v + w * w;
+    float n2 = W ? fmaf(w, w, sum_sq<W>(u, v)) : u * u + v * v + w * w;
     if (n2 > 0.f && fabsf(n2 - 1.f) > 1e-6f) {
 #ifdef __CUDA_ARCH__
         float r = rsqrtf(n2);
@@ -242,9 +261,9 @@ struct Uphi {
     R A, B, C, cphi, sphi;
 };
 
-template <typename R>
+template <typename R, bool PIN = false>
 OMC_HD void rotate_into(R A, R B, R C, R costhe, R sinthe, R cphi, R sphi, R &u, R &v, R &w) {
-    R sinps2 = A * A + B * B;
+    R sinps2 = sum_sq<PIN ? 1 : 0>(A, B);
     if (sinps2 < R(1.0E-20)) {
         u = sinthe * cphi;
         v = sinthe * sphi;
@@ -265,8 +284,8 @@ template <typename R, typename Env>
 OMC_HD void uphi21(Env &g, Part<R> &p, Uphi<R> &h, R costhe, R sinthe) {
     azimuth(g, h.cphi, h.sphi);
     h.A = p.u; h.B = p.v; h.C = p.w;
-    rotate_into(h.A, h.B, h.C, costhe, sinthe, h.cphi, h.sphi, p.u, p.v, p.w);
-    renorm_dir(p.u, p.v, p.w);
+    rotate_into<R, BufferedRng<Env>::value>(h.A, h.B, h.C, costhe, sinthe, h.cphi, h.sphi, p.u, p.v, p.w);
+    renorm_dir<BufferedRng<Env>::value ? 1 : 0>(p.u, p.v, p.w);
 }
 
 // Partner particle: position, region and weight of p, direction rotated
@@ -1402,10 +1421,10 @@ OMC_HD R msdist(const DevData<R> &D, Env &g, const Part<R> &p, int imed, int iq,
         }
     }
     R u2 = sint2 * cphi2, v2 = sint2 * sphi2;
-    R u2p = w1 * u2 + sint1 * w2;
-    R us = u2p * cphi1 - v2 * sphi1;
-    R vs = u2p * sphi1 + v2 * cphi1;
-    R ws = w1 * w2 - sint1 * u2;
+    R u2p = sum_fma2(w1, u2, sint1, w2);
+    R us = sum_fma1(u2p, cphi1, -v2, sphi1);
+    R vs = sum_fma2(u2p, sphi1, v2, cphi1);
+    R ws = sum_fma1(w1, w2, -sint1, u2);
     xi *= R(2) * xi_corr;
     R eta = g.uni();
     R eta1 = R(0.5) * (R(1) - eta);
@@ -1425,15 +1444,15 @@ OMC_HD R msdist(const DevData<R> &D, Env &g, const Part<R> &p, int imed, int iq,
     R wt = eta1 * (R(1) + temp) + b * w1 + c * w2 + eta1 * ws * temp1;
     R ustep = tustep * m_sqrt(ut * ut + vt * vt + wt * wt);
     R u0 = p.u, v0 = p.v, w0 = p.w;
-    R sint02 = u0 * u0 + v0 * v0;
+    R sint02 = sum_sq<1>(u0, v0);
     if (sint02 > R(1.0E-20)) {
         R sint0 = m_sqrt(sint02);
         R sint0i = R(1) / sint0;
         R cphi0 = sint0i * u0, sphi0 = sint0i * v0;
-        u2p = w0 * us + sint0 * ws;
-        ws = w0 * ws - sint0 * us;
-        us = u2p * cphi0 - vs * sphi0;
-        vs = u2p * sphi0 + vs * cphi0;
+        u2p = sum_fma1(w0, us, sint0, ws);
+        ws = sum_fma1(w0, ws, -sint0, us);
+        us = sum_fma1(u2p, cphi0, -vs, sphi0);
+        vs = sum_fma1(u2p, sphi0, vs, cphi0);
         u2p = w0 * ut + sint0 * wt;
         wt = w0 * wt - sint0 * ut;
         ut = u2p * cphi0 - vt * sphi0;
@@ -1792,7 +1811,7 @@ OMC_HD int electron_transport(const DevData<R> &D, Env &g, Part<R> &p, R &edep_e
             g.deposit(p.ir, p.wt * edep);
             p.x = xf; p.y = yf; p.z = zf;
             p.u = uf; p.v = vf; p.w = wf;
-            renorm_dir(p.u, p.v, p.w);
+            renorm_dir<2>(p.u, p.v, p.w);
             irold = p.ir;
             eie -= edep;
             p.e = eie;

@@ -79,6 +79,7 @@ struct Philox {
             ctr++;
         }
     }
+    OMC_HD uint64_t key() const { return ((uint64_t)k1 << 32) | k0; }
     // Numbers drawn so far (the argument init() resumes from).
     OMC_HD uint32_t position() const { return (ctr << 2) - 4u + (uint32_t)pos; }
     // The block generator runs once per four numbers.
