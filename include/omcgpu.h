@@ -94,7 +94,8 @@ typedef struct {
     int profile;          /* 1: event form launches cycles one by one and times
                              every kernel (see omc_profile_last) */
     int electron_tsteps;  /* event form: tstep-loop iterations an electron runs
-                             per launch before it is re-queued (0 = default 1) */
+                             per launch before it is re-queued (0 = default: 2,
+                             1 in the FP64 event form) */
     int64_t inflight;     /* event form: particles kept in flight (0 = default) */
     int tail_boost;       /* event form: largest factor by which event budgets
                              grow as the queues drain (0 = default 32, 1 = fixed
@@ -122,8 +123,9 @@ typedef struct {
                              at most this many particles are left, they are
                              run to the end of their sub-histories in one
                              launch instead of further cycles (0 = default,
-                             half of the drain kernel's resident threads;
-                             -1 = never);
+                             one and a half times the drain kernel's resident
+                             threads, once them when photons are split, half
+                             of them in the FP64 event form; -1 = never);
                              results do not depend on it */
 } omc_options;
 

@@ -669,7 +669,8 @@ __global__ void __launch_bounds__(EV_MAX_BLOCK) k_electron_interact(DevData<R> D
 // tickets below the number of queued particles are those, the others wait
 // for the pool entry of their number to be marked ready, or for the end.
 // A lane donates only while tickets outnumber entries (compare and swap), so
-// an entry always has a taker.  The launch is over when as many tasks are
+// an entry has a taker at once; one that a full stack puts there waits for the
+// next warp without work.  The launch is over when as many tasks are
 // done as were made.  Lanes wait only when no particle is left unclaimed, so
 // blocks that are not resident yet hold nobody up, and every wait has a
 // limit.
@@ -804,6 +805,16 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
     unsigned c_ev[2] = {0, 0}, c_steps[2] = {0, 0}, c_cross[2] = {0, 0}, c_dep[2] = {0, 0}, c_atom = 0;
     int x_ev = 0, x_chain = 0, x_steps = 0;   // this task: events, events of its first particle, steps
     int first_at = 0;                         // where the first particle is: stack entry, -1 in hand, -2 gone
+    // the oldest pending particle into pool entry k
+    auto give = [&](int k) {
+        const DrainPart<R> &e = st[0];
+        qstore(pool, k, e.p, g.slot, e.k0, e.k1, e.pos, e.sp, e.sr);
+        depth--;
+        for (int i = 0; i < depth; i++) st[i] = st[i + 1];
+        first_at = first_at == 0 ? -2 : (first_at > 0 ? first_at - 1 : first_at);
+        __threadfence();
+        *(volatile int *)&ready[k] = 1;
+    };
     for (int idle = 0;;) {
         // the warps of a block take their iterations, and the phases of an
         // iteration, together, so that they share the instructions they fetch
@@ -943,8 +954,14 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
                                       ((uint64_t)k << 40));
             if (alive) {
                 if (depth >= DRAIN_STACK) {
-                    g.flags |= ERR_STACK;
-                    continue;
+                    // a full stack hands its oldest particle over, asked or
+                    // not (deep cascades of split rays)
+                    const int k2 = atomicAdd(&ctl->drain_tail, 1);
+                    if (k2 >= pool_cap) {
+                        g.flags |= ERR_STACK;
+                        continue;
+                    }
+                    give(k2);
                 }
                 const uint64_t key = g.rng.key();
                 st[depth].p = p;
@@ -985,18 +1002,14 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
             if (tail < pool_cap && ld_volatile(&ctl->drain_head) > n + tail &&
                 atomicCAS(&ctl->drain_tail, tail, tail + 1) == tail) {
                 if (depth > 0) {
-                    const DrainPart<R> &e = st[0];
-                    qstore(pool, tail, e.p, g.slot, e.k0, e.k1, e.pos, e.sp, e.sr);
-                    depth--;
-                    for (int i = 0; i < depth; i++) st[i] = st[i + 1];
-                    first_at = first_at == 0 ? -2 : (first_at > 0 ? first_at - 1 : first_at);
+                    give(tail);
                 } else {
                     const uint64_t key = g.rng.key();
                     qstore(pool, tail, p, g.slot, (uint32_t)key, (uint32_t)(key >> 32), g.rng.position(), sp, sr);
                     alive = false;
+                    __threadfence();
+                    *(volatile int *)&ready[tail] = 1;
                 }
-                __threadfence();
-                *(volatile int *)&ready[tail] = 1;
             }
         }
         if (!alive) {
@@ -1313,6 +1326,17 @@ static int event_interact_queue_t(omc_engine *e) {
 }
 int event_interact_queue(omc_engine *e) { return event_interact_queue_t<float>(e); }
 
+// Electron budget of an event: tstep-loop iterations, of electron_chsteps
+// condensed-history steps each, while the queue fills the GPU.  Lanes of a
+// warp that go on together do similar work, but every event costs a round
+// trip through the queue.  FP32: 1 / 2 / 3 iterations 100.3 / 98.4 / 108.1 ms
+// on the slab beam (1e7 histories), 103.8 / 94.4 / 92.9 ms on the 200^3-class
+// 18 MV beam (1e6).
+template <typename R>
+static int default_tsteps() {
+    return sizeof(R) == 4 ? 2 : 1;
+}
+
 template <typename R>
 static int event_prepare_t(omc_engine *e) {
     EventStateT<R> *&sp = state_of<R>(e);
@@ -1326,9 +1350,7 @@ static int event_prepare_t(omc_engine *e) {
     S.block = e->opt.block > 0 ? std::min(EV_MAX_BLOCK, (e->opt.block + 31) / 32 * 32) : 256;
     S.grid = e->sm_count * std::max(1, 2048 / S.block);
     size_grids(e, S);
-    // 1 measured best on the slab workload while the queues are full (with
-    // the default electron_chsteps = 3: at most three CH steps per event)
-    S.tsteps = e->opt.electron_tsteps > 0 ? e->opt.electron_tsteps : 1;
+    S.tsteps = e->opt.electron_tsteps > 0 ? e->opt.electron_tsteps : default_tsteps<R>();
     S.boost = e->opt.tail_boost > 0 ? e->opt.tail_boost : 32;
     S.inflight = e->opt.inflight > 0 ? e->opt.inflight : (1LL << 20);
     S.esplit = e->opt.electron_split > 0 ? e->opt.electron_split + D_RM : 0.0;
@@ -1348,6 +1370,10 @@ static int event_prepare_t(omc_engine *e) {
             q.sr = (float *)((char *)S.split_buf[k].p + per);
         }
     }
+    if (cudaHostAlloc((void **)&S.snap, 2 * sizeof(Ctl), cudaHostAllocDefault) != cudaSuccess ||
+        cudaEventCreateWithFlags(&S.snap_ev[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&S.snap_ev[1], cudaEventDisableTiming) != cudaSuccess)
+        return set_err(e, OMC_E_DEVICE, "control block snapshots");
     if (cudaStreamCreateWithFlags(&S.side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&S.fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&S.join, cudaEventDisableTiming) != cudaSuccess)
@@ -1410,7 +1436,8 @@ int event_set_params(omc_engine *e, int tsteps, int boost, long long inflight, i
         e->opt.block = block;
     }
     auto apply = [&](auto &S) {
-        S.tsteps = e->opt.electron_tsteps > 0 ? e->opt.electron_tsteps : 1;
+        using R = decltype(S.q[0].pos->x);
+        S.tsteps = e->opt.electron_tsteps > 0 ? e->opt.electron_tsteps : default_tsteps<R>();
         S.boost = e->opt.tail_boost > 0 ? e->opt.tail_boost : 32;
         S.inflight = e->opt.inflight > 0 ? e->opt.inflight : (1LL << 20);
         S.esplit = e->opt.electron_split > 0 ? e->opt.electron_split + D_RM : 0.0;
@@ -1447,10 +1474,10 @@ void event_release(omc_engine *e) {
 
 // One transport cycle with input buffers `in` (0 = A, 1 = B).  With `ev`
 // (profiling) the launches are sequential and an event is recorded before
-// each and after the last.
+// each and after the last.  source = false: a cycle after the last injection.
 template <typename R = float>
 static void launch_cycle(omc_engine *e, int in, const BeamSrc<R> &src, double *tallies, long nper, uint64_t seed,
-                         long long target, cudaEvent_t *ev = nullptr) {
+                         long long target, cudaEvent_t *ev = nullptr, bool source = true) {
     EventStateT<R> &S = *state_of<R>(e);
     int iph = in == 0 ? 0 : 2, iel = iph + 1;
     int oph = in == 0 ? 2 : 0, oel = oph + 1;
@@ -1458,24 +1485,30 @@ static void launch_cycle(omc_engine *e, int in, const BeamSrc<R> &src, double *t
     if (ev) cudaEventRecord(ev[0], e->stream);
     k_plan<<<1, 1, 0, e->stream>>>(S.ctl_d, iph, iel, plan_cfg_t<R>(e, target));
     if (ev) cudaEventRecord(ev[1], e->stream);
-    k_source<R><<<S.grid, S.block, 0, e->stream>>>(event_data<R>(e), src, S.q[iph], S.q[iel], S.ctl_d, nper, seed,
-                                                   seedw);
+    if (source)
+        k_source<R><<<S.grid, S.block, 0, e->stream>>>(event_data<R>(e), src, S.q[iph], S.q[iel], S.ctl_d, nper, seed,
+                                                       seedw);
     if (ev) cudaEventRecord(ev[2], e->stream);
     launch_transport<R>(e, iph, iel, oph, oel, tallies, seedw, nullptr, 1, ev);
     if (ev) cudaEventRecord(ev[4], e->stream);
 }
 
 // Particles left in the queues at or below which the transport switches
-// from cycles to the drain (0: never).  By default half of the drain
-// kernel's resident threads (≈38 k): the drain serialises each particle's
-// whole remaining cascade in one thread, so it pays only once the cycles
-// are mostly idle (measured on slab64: ≈40 k best of 5 k - 1 M particles,
-// for 10^6- and 10^7-history runs alike).
+// from cycles to the drain (0: never).  The drain spreads its particles over the GPU, so it takes
+// over once a cycle is shorter than one wave of the electron kernel: one and
+// a half times its resident threads (114 k; the slab beam of 1e6 histories
+// took 26.1 / 25.4 / 25.0 / 25.0 / 25.2 ms from 38 / 75 / 110 / 200 / 300 k
+// on); with photon splitting, whose rays a lane works off one sub-photon
+// after the other, once them (water phantom, 124 k histories split in 20:
+// 63.5 / 61.6 / 75.4 ms from 38 / 75 / 113 k on).  The FP64 form's runs one
+// particle a thread: half of them.
 template <typename R>
 static long long drain_threshold_t(const omc_engine *e) {
     const EventStateT<R> &S = state<R>(e);
     if (e->opt.drain_particles < 0) return 0;
-    return e->opt.drain_particles > 0 ? e->opt.drain_particles : S.drain_lanes / 2;
+    if (e->opt.drain_particles > 0) return e->opt.drain_particles;
+    if (sizeof(R) == 8) return S.drain_lanes / 2;
+    return e->d32.d.nsplit > 1 ? S.drain_lanes : (long long)S.drain_lanes * 3 / 2;
 }
 long long drain_threshold(const omc_engine *e) { return drain_threshold_t<float>(e); }
 
@@ -1607,8 +1640,7 @@ int event_run_beam(omc_engine *e, const omc_beam *b, long nper, int nbatch, uint
         cudaEventCreate(&t1);
         cudaEventRecord(t0, e->stream);
         if constexpr (sizeof(R) == 4) rc = run_profiled(e, src, tal.as<double>(), nper, seed, target, h, cycles);
-        for (int ib = 0; ib < nbatch && rc == OMC_OK; ib++)
-            rc = fold(e, tal.as<double>() + (size_t)ib * nvox, sum, sum2, nvox, 1.0);
+        if (!rc) rc = fold(e, tal.as<double>(), nbatch, sum, sum2, nvox, 1.0);
         cudaEventRecord(t1, e->stream);
         cudaEventSynchronize(t1);
         float ms = 0;
@@ -1616,7 +1648,7 @@ int event_run_beam(omc_engine *e, const omc_beam *b, long nper, int nbatch, uint
         cudaEventDestroy(t0);
         cudaEventDestroy(t1);
         ks.seconds = ms * 1e-3;
-        ks.launches = cycles * (e->d32.d.defer_interact ? 5 : 4) + nbatch + (drain_threshold(e) > 0 ? 1 : 0);
+        ks.launches = cycles * (e->d32.d.defer_interact ? 5 : 4) + 1 + (drain_threshold(e) > 0 ? 1 : 0);
         ks.flags |= h.flags;
         for (int k = 0; k < 2; k++) {
             KernelProfile &P = S.prof[1 + k];
@@ -1632,77 +1664,121 @@ int event_run_beam(omc_engine *e, const omc_beam *b, long nper, int nbatch, uint
         return OMC_OK;
     }
 
-    // capture two cycles (A -> B, B -> A) as one graph
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    if ((rc = cuda_check(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal), "capture"))) return rc;
-    launch_cycle<R>(e, 0, src, tal.as<double>(), nper, seed, target);
-    launch_cycle<R>(e, 1, src, tal.as<double>(), nper, seed, target);
-    if ((rc = cuda_check(e, cudaStreamEndCapture(e->stream, &graph), "end capture"))) return rc;
-    if ((rc = cuda_check(e, cudaGraphInstantiate(&exec, graph, 0), "graph instantiate"))) {
-        cudaGraphDestroy(graph);
-        return rc;
-    }
     cudaEvent_t t0, t1;
     cudaEventCreate(&t0);
     cudaEventCreate(&t1);
-    cudaEventRecord(t0, e->stream);
     Ctl h{};
-    long graphs = 0;
-    int per_check = 4;
+    long launches = 0;
+    const uint32_t seedw = (uint32_t)(seed >> 32);
+    const int cycle_launches = e->d32.d.defer_interact ? 5 : 4;
     const long long dthr = drain_threshold_t<R>(e);
-    int drains = 0;
-    for (;;) {
-        for (int k = 0; k < per_check; k++) cudaGraphLaunch(exec, e->stream);
-        graphs += per_check;
-        cudaMemcpyAsync(&h, S.ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost, e->stream);
-        if ((rc = cuda_check(e, cudaStreamSynchronize(e->stream), "event transport"))) break;
-        // a graph ends with a B -> A cycle: its outputs are queues A
-        if (h.hist_next >= h.hist_total && h.cnt[0] == 0 && h.cnt[1] == 0 && h.cnt_hi[0] == 0 &&
-            h.cnt_hi[1] == 0)
-            break;
-        if (h.flags & ERR_QUEUE) break;
-        if (dthr > 0 && h.hist_next >= h.hist_total) {
-            // every history is in: drain once few particles are left,
-            // checking after every graph until then
-            long long left = (long long)std::min(h.cnt[0] + h.cnt_hi[0], S.cap) +
-                             std::min(h.cnt[1] + h.cnt_hi[1], S.cap);
-            if (left <= dthr) {
-                launch_drain<R>(e, 0, left, tal.as<double>(), (uint32_t)(seed >> 32));
-                drains = 1;
-                if ((rc = cuda_check(e, cudaStreamSynchronize(e->stream), "drain"))) break;
-                cudaMemcpy(&h, S.ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost);
+    const int pweight = plan_cfg_t<R>(e, target).pweight;
+    // A run whose histories the drain's warps hold at once goes to the drain
+    // as it is (10^4 histories on the water phantom 8.4 -> 4.1 ms, 3 10^4
+    // 8.9 -> 5.4, 10^5 no gain).
+    const bool direct = sizeof(R) == 4 && pweight == 1 &&
+                        c0.hist_total <= std::min({dthr, (long long)S.drain_lanes / 2, target});
+    // two cycles (A -> B, B -> A) as one graph, and two without injection
+    cudaGraph_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    auto capture = [&](int k) {
+        int r = cuda_check(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal), "capture");
+        if (r) return r;
+        for (int in = 0; in < 2; in++)
+            launch_cycle<R>(e, in, src, tal.as<double>(), nper, seed, target, nullptr, k == 0);
+        if ((r = cuda_check(e, cudaStreamEndCapture(e->stream, &graph[k]), "end capture"))) return r;
+        return cuda_check(e, cudaGraphInstantiate(&exec[k], graph[k], 0), "graph instantiate");
+    };
+    auto queued = [&](const Ctl &c) {   // a graph ends with a B -> A cycle: its outputs are queues A
+        return (long long)std::min(c.cnt[0] + c.cnt_hi[0], S.cap) + std::min(c.cnt[1] + c.cnt_hi[1], S.cap);
+    };
+    cudaEventRecord(t0, e->stream);
+    long long left = 0;   // particles for the drain, at most
+    if (direct) {
+        k_plan<<<1, 1, 0, e->stream>>>(S.ctl_d, 0, 1, plan_cfg_t<R>(e, target));
+        k_source<R><<<S.grid, S.block, 0, e->stream>>>(event_data<R>(e), src, S.q[0], S.q[1], S.ctl_d, nper, seed,
+                                                       seedw);
+        launches += 2;
+        left = c0.hist_total;
+    } else if (!(rc = capture(0))) {
+        // Checked after every graph where the end is near: from the start on
+        // when one cycle injects all (with splitting, where the drain's lanes
+        // hold all sub-photons: 10^3 histories split in 20 15.7 -> 11.1 ms, but
+        // 10^4 18.9 -> 26.5).
+        const long long few = pweight == 1 ? target : S.drain_lanes;
+        int per_check = sizeof(R) == 4 && c0.hist_total * pweight <= few ? 1 : 4;
+        for (long graphs = 0;;) {
+            for (int k = 0; k < per_check; k++) cudaGraphLaunch(exec[0], e->stream);
+            graphs += per_check;
+            launches += per_check * 2 * cycle_launches;
+            cudaMemcpyAsync(S.snap, S.ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost, e->stream);
+            if ((rc = cuda_check(e, cudaStreamSynchronize(e->stream), "event transport"))) break;
+            h = S.snap[0];
+            left = queued(h);
+            if ((h.hist_next >= h.hist_total && left == 0) || (h.flags & ERR_QUEUE)) break;
+            if (dthr > 0 && h.hist_next >= h.hist_total) {
+                if (sizeof(R) == 4 || left <= dthr) break;
+                per_check = 1;
+                continue;
+            }
+            // every cycle advances each queued particle by one event, so a run
+            // needs (histories / injection rate) + (longest history) cycles
+            if (graphs > 50000 + h.hist_total / 1000) {
+                rc = set_err(e, OMC_E_DEVICE, "event transport did not drain");
                 break;
             }
-            per_check = 1;
-            continue;
+            per_check = std::min(per_check * 2, 64);
+            if (sizeof(R) == 4 && h.hist_next < h.hist_total)
+                per_check = (int)std::max(1.0, std::min<double>(per_check, 0.5 * graphs * (h.hist_total - h.hist_next) /
+                                                                               std::max<long long>(h.hist_next, 1)));
         }
-        // every cycle advances each queued particle by one event, so a run
-        // needs (histories / injection rate) + (longest history) cycles
-        if (graphs > 50000 + h.hist_total / 1000) {
-            rc = set_err(e, OMC_E_DEVICE, "event transport did not drain");
-            break;
+        // FP32, every history injected: cycles without the source kernel, the
+        // next pair queued before the last one's state is looked at
+        if (sizeof(R) == 4 && !rc && dthr > 0 && left > dthr && !(h.flags & ERR_QUEUE) && !(rc = capture(1))) {
+            for (long graphs = 0;; graphs++) {
+                cudaGraphLaunch(exec[1], e->stream);
+                launches += 2 * (cycle_launches - 1);
+                const int k = graphs & 1;
+                cudaMemcpyAsync(&S.snap[k], S.ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost, e->stream);
+                cudaEventRecord(S.snap_ev[k], e->stream);
+                if (graphs == 0) continue;
+                if ((rc = cuda_check(e, cudaEventSynchronize(S.snap_ev[k ^ 1]), "event transport"))) break;
+                h = S.snap[k ^ 1];
+                left = queued(h);
+                if (left <= dthr || (h.flags & ERR_QUEUE)) break;
+                if (graphs > 100000) {
+                    rc = set_err(e, OMC_E_DEVICE, "event transport did not drain");
+                    break;
+                }
+            }
         }
-        per_check = std::min(per_check * 2, 64);
+    }
+    if (!rc && left > 0 && dthr > 0 && !(h.flags & ERR_QUEUE)) {
+        launch_drain<R>(e, 0, left, tal.as<double>(), seedw);
+        launches++;
     }
     // fold the batch tallies into the sums (accumEndep per batch)
-    for (int ib = 0; ib < nbatch && rc == OMC_OK; ib++)
-        rc = fold(e, tal.as<double>() + (size_t)ib * nvox, sum, sum2, nvox, 1.0);
+    if (!rc) rc = fold(e, tal.as<double>(), nbatch, sum, sum2, nvox, 1.0);
     cudaEventRecord(t1, e->stream);
-    cudaEventSynchronize(t1);
-    float ms = 0;
-    cudaEventElapsedTime(&ms, t0, t1);
-    ks.seconds = ms * 1e-3;
-    ks.launches = graphs * (e->d32.d.defer_interact ? 10 : 8) + nbatch + drains;
-    ks.flags |= h.flags;
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
+    // source energy, and the error flags of all that ran
+    cudaMemcpyAsync(src_energy, &S.ctl_d->src_energy, 8, cudaMemcpyDeviceToDevice, e->stream);
+    cudaMemcpyAsync(S.snap, S.ctl_d, sizeof(Ctl), cudaMemcpyDeviceToHost, e->stream);
+    const int sync = cuda_check(e, cudaStreamSynchronize(e->stream), "event transport");
+    if (!rc) rc = sync;
+    if (!rc) {
+        float ms = 0;
+        cudaEventElapsedTime(&ms, t0, t1);
+        ks.seconds = ms * 1e-3;
+        ks.launches = launches + 1;
+        ks.flags |= S.snap[0].flags;
+    }
+    for (int k = 0; k < 2; k++) {
+        if (exec[k]) cudaGraphExecDestroy(exec[k]);
+        if (graph[k]) cudaGraphDestroy(graph[k]);
+    }
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
-    if (rc) return rc;
-    // source energy
-    cudaMemcpyAsync(src_energy, &S.ctl_d->src_energy, 8, cudaMemcpyDeviceToDevice, e->stream);
-    return OMC_OK;
+    return rc;
 }
 template int event_run_beam<float>(omc_engine *, const omc_beam *, long, int, uint64_t, double *, double *, double *,
                                    KernelStats &);

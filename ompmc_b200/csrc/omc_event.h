@@ -119,7 +119,13 @@ struct EventStateT {
     // beside the electron kernels of its cycle (fork/join events)
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    // control block as the host last saw it (pinned), two of them in turn
+    Ctl *snap = nullptr;
+    cudaEvent_t snap_ev[2] = {nullptr, nullptr};
     ~EventStateT() {
+        for (auto ev : snap_ev)
+            if (ev) cudaEventDestroy(ev);
+        if (snap) cudaFreeHost(snap);
         if (fork) cudaEventDestroy(fork);
         if (join) cudaEventDestroy(join);
         if (side) cudaStreamDestroy(side);
@@ -178,5 +184,5 @@ int event_run_beam(omc_engine *e, const omc_beam *b, long nper, int nbatch, uint
 void event_release(omc_engine *e);
 template <typename R>
 BeamSrc<R> beam_setup(const omc_engine *e, const omc_beam *b);
-int fold(omc_engine *e, double *work, double *sum, double *sum2, long n, double scale);
+int fold(omc_engine *e, double *work, int nb, double *sum, double *sum2, long n, double scale);
 }  // namespace omc

@@ -147,9 +147,8 @@ extern "C" int omc_run_beam_noalloc(omc_engine *e, const omc_beam *b, int64_t nc
         if ((rc = plain_beam_batches(e, S, work, seed, (long)b0 * nper, nb, nper, (unsigned long long *)(acc + 2),
                                      acc + 1, block, &launches)))
             return rc;
-        for (int ib = 0; ib < nb; ib++)
-            if ((rc = fold(e, work + (long)ib * nv, sum, sum2, nv, 1.0))) return rc;
-        launches += nb;
+        if ((rc = fold(e, work, nb, sum, sum2, nv, 1.0))) return rc;
+        launches++;
     }
     if ((rc = device_sum(e, sum, nv, acc))) return rc;
     if ((rc = finalize_dosxyz(e, sum, sum2, nbatch, (double)nper, dose_d, unc_d))) return rc;

@@ -21,7 +21,10 @@ FORMS = [dict(drain_particles=-1), dict(), dict(drain_particles=1 << 22), dict(d
     ("slab", dict(mono_energy=6.0), 1, 20), ("slab", dict(mono_energy=6.0), 1, 2400),
     ("ct", dict(mono_energy=12.0), 1, 60_000), ("ct", dict(mono_energy=4.0, charge=1), 1, 3000),
     ("slab", dict(mono_energy=8.0, charge=-1), 1, 37), ("slab", dict(mono_energy=5.0), 5, 5000),
-    ("ct", dict(mono_energy=10.0), 20, 500)])
+    ("ct", dict(mono_energy=10.0), 20, 500),
+    # cascades of split rays deeper than a lane's stack (bremsstrahlung and
+    # scattered photons of 18 MeV photons in water)
+    ("water", dict(mono_energy=18.0), 64, 3000)])
 def test_dose_independent_of_where_particles_run(kind, source, nsplit, histories):
     from ompmc_b200.engine import EVENT_FP32, Engine
     ph = cases._phantom(kind, 32, 5.0)
