@@ -7,6 +7,8 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <system_error>
+#include <thread>
 
 #include "omc_engine.h"
 #include "omc_event.h"
@@ -391,6 +393,65 @@ template BeamSrc<float> beam_setup<float>(const omc_engine *, const omc_beam *);
 
 }  // namespace omc
 
+// A large result into the caller's pageable memory: RESULT_THREADS threads take
+// its chunks in turn, each through two pinned buffers of its own, so that the
+// transfer, the copies and the first touch of the caller's pages overlap (one
+// copy after the other by the driver moved some 6 GB/s).
+namespace {
+constexpr size_t RESULT_CHUNK = (size_t)1 << 20, RESULT_STAGED = (size_t)8 << 20;
+constexpr int RESULT_THREADS = 4;
+
+int fetch_result(omc_engine *e, void *dst, const void *src, size_t bytes) {
+    cudaPointerAttributes at{};
+    const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    if (bytes < RESULT_STAGED || pinned)
+        return cuda_check(e, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, e->stream), "d2h");
+    if (!e->result_stage &&
+        cudaHostAlloc(&e->result_stage, 2 * RESULT_THREADS * RESULT_CHUNK, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        e->result_stage = nullptr;
+        return cuda_check(e, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, e->stream), "d2h");
+    }
+    const size_t chunks = (bytes + RESULT_CHUNK - 1) / RESULT_CHUNK;
+    std::atomic<int> failed{0};
+    auto work = [&](int t) {
+        cudaSetDevice(e->device);
+        cudaEvent_t ev[2] = {nullptr, nullptr};
+        cudaError_t rc = cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
+        if (rc == cudaSuccess) rc = cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming);
+        char *stage = (char *)e->result_stage + (size_t)t * 2 * RESULT_CHUNK;
+        auto size = [&](size_t c) { return std::min(RESULT_CHUNK, bytes - c * RESULT_CHUNK); };
+        auto issue = [&](size_t c, int k) {
+            if (rc == cudaSuccess && c < chunks) {
+                rc = cudaMemcpyAsync(stage + k * RESULT_CHUNK, (const char *)src + c * RESULT_CHUNK, size(c),
+                                     cudaMemcpyDeviceToHost, e->stream);
+                if (rc == cudaSuccess) rc = cudaEventRecord(ev[k], e->stream);
+            }
+        };
+        issue(t, 0);
+        int k = 0;
+        for (size_t c = t; c < chunks && rc == cudaSuccess; c += RESULT_THREADS, k ^= 1) {
+            issue(c + RESULT_THREADS, k ^ 1);
+            if (rc == cudaSuccess) rc = cudaEventSynchronize(ev[k]);
+            if (rc == cudaSuccess) std::memcpy((char *)dst + c * RESULT_CHUNK, stage + k * RESULT_CHUNK, size(c));
+        }
+        for (auto x : ev)
+            if (x) cudaEventDestroy(x);
+        if (rc != cudaSuccess) failed = (int)rc;
+    };
+    std::vector<std::thread> pool;
+    int rest = 1;   // stripes that have no thread are done here, after our own
+    try {
+        for (; rest < RESULT_THREADS; rest++) pool.emplace_back(work, rest);
+    } catch (const std::system_error &) {
+    }
+    work(0);
+    for (; rest < RESULT_THREADS; rest++) work(rest);
+    for (auto &t : pool) t.join();
+    return failed ? cuda_check(e, (cudaError_t)(int)failed, "d2h") : OMC_OK;
+}
+}  // namespace
+
 // =================================================================== C ABI
 extern "C" {
 
@@ -595,6 +656,7 @@ int omc_engine_destroy(omc_engine *e) {
     cudaSetDevice(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
     event_release(e);
+    if (e->result_stage) cudaFreeHost(e->result_stage);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
     return OMC_OK;
@@ -724,8 +786,8 @@ int omc_run_beam(omc_engine *e, const omc_beam *b, int64_t ncase, int nbatch, ui
     unsigned flags = 0;
     if ((rc = cuda_check(e, cudaMemcpyAsync(accum, acc.p, 4 * 8, cudaMemcpyDeviceToHost, e->stream), "d2h"))) return rc;
     cudaMemcpyAsync(&flags, e->errword.p, sizeof(unsigned), cudaMemcpyDeviceToHost, e->stream);
-    if (dose) cudaMemcpyAsync(dose, out_d.p, nv * 8, cudaMemcpyDeviceToHost, e->stream);
-    if (unc) cudaMemcpyAsync(unc, unc_d.p, nv * 8, cudaMemcpyDeviceToHost, e->stream);
+    if (dose && (rc = fetch_result(e, dose, out_d.p, nv * 8))) return rc;
+    if (unc && (rc = fetch_result(e, unc, unc_d.p, nv * 8))) return rc;
     if ((rc = cuda_check(e, cudaStreamSynchronize(e->stream), "beam results"))) return rc;
     ks.flags |= flags;
     if (stats) {

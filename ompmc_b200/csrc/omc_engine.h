@@ -89,6 +89,7 @@ struct omc_engine {
     std::string err;
     std::vector<double> mass;  // voxel mass (g), host copy
     omc::DBuf mass_d;
+    void *result_stage = nullptr;   // pinned buffers large results pass through
     // device buffers of omc_run_beam, kept between calls and grown on
     // demand so that a run allocates nothing once the engine is warm
     omc::DBuf run_sum, run_sum2, run_out, run_unc, run_acc, run_cdf, run_work, run_tal, run_cdf32;

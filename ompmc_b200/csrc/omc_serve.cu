@@ -259,6 +259,25 @@ int check_beamlets(omc_engine *e, const omc_beamlets *b) {
     return OMC_OK;
 }
 
+// Results are written once, so their storage need not be cleared first.
+template <typename T>
+struct Uninit : std::allocator<T> {
+    template <typename U>
+    struct rebind {
+        using other = Uninit<U>;
+    };
+    template <typename U>
+    void construct(U *p) {
+        ::new ((void *)p) U;
+    }
+    template <typename U, typename... A>
+    void construct(U *p, A &&...a) {
+        ::new ((void *)p) U(std::forward<A>(a)...);
+    }
+};
+template <typename T>
+using Result = std::vector<T, Uninit<T>>;
+
 struct Request {
     int id = -1, kind = 0, slot = -1, state = 0;  // state 0 pending, 1 running, 2 done, 3 released
     long long nhist = 0, nper = 0;
@@ -269,8 +288,8 @@ struct Request {
     omc_beam beam{};
     DBuf cdf;
     double t_submit = 0, t_done = 0;
-    std::vector<int32_t> rows;
-    std::vector<double> vals, var, dose, unc;
+    Result<int32_t> rows;
+    Result<double> vals, var, dose, unc;
     uint64_t seed = 0;
 };
 
@@ -330,27 +349,44 @@ struct omc_server {
         }
         for (auto &sn : snap)
             if (sn.ev) cudaEventDestroy(sn.ev);
+        for (auto &f : fbuf)
+            if (f.ev) cudaEventDestroy(f.ev);
+        if (copy_stream) {
+            cudaStreamSynchronize(copy_stream);
+            cudaStreamDestroy(copy_stream);
+        }
         if (snap_host) cudaFreeHost(snap_host);
     }
     // state after the last step: particles in the queues, and whether every
     // running request had all its histories injected
     long long left = 0;
     bool injected = false;
-    // finalise scratch (device): sum, sum2, dose, var | rows | vals | vars | seg counts/offsets | dmax | total
-    double *f_sum = nullptr, *f_sum2 = nullptr, *f_dose = nullptr, *f_var = nullptr, *f_vals = nullptr,
-           *f_vars = nullptr;
-    int *f_rows = nullptr, *f_cnt = nullptr, *f_off = nullptr;
-    unsigned long long *f_dmax = nullptr;
-    long long *f_total = nullptr;
+    // Finalisation of finished requests, two at a time: device scratch (dose,
+    // var, column values, variances, rows | segment counts, offsets | column
+    // maximum, entries), and where the host takes the column over (pinned)
+    struct Fin {
+        double *dose = nullptr, *var = nullptr, *vals = nullptr, *vars = nullptr;
+        int *rows = nullptr, *cnt = nullptr, *off = nullptr;
+        unsigned long long *dmax = nullptr;
+        long long *total = nullptr;
+        long long *total_h = nullptr;
+        char *stage = nullptr;
+        cudaEvent_t ev = nullptr;
+    } fbuf[2];
+    cudaStream_t copy_stream = nullptr;
 };
 
 namespace {
 
-// Fold, finalise and extract one finished request into host memory, on the
+// Column bytes (row, value and variance of each entry) that the pinned
+// staging buffers hold; longer columns go straight to the request's arrays.
+constexpr size_t FIN_STAGE = (size_t)3 << 19;
+
+// Fold, finalise and extract one finished request on the device, on the
 // finalisation stream (the transport work queued on the engine's stream
 // goes on meanwhile; it does not touch this request's tallies, whose live
 // count is zero and whose histories are all injected).
-int finalize_request(omc_server *s, Request &r) {
+int finalize_launch(omc_server *s, const Request &r, omc_server::Fin &f) {
     omc_engine *e = s->e;
     cudaStream_t st = s->fin_stream;
     long nv = e->ph.nvox();
@@ -359,37 +395,59 @@ int finalize_request(omc_server *s, Request &r) {
     s->launches += r.kind == 0 ? 1 : 4;   // fused fold + finalise (+ column extraction)
     double *tal = s->tallies.as<double>() + (size_t)r.slot * s->nbmax * nv;
     int g = std::max(1, std::min((int)((nv + 255) / 256), e->sm_count * 8));
-    if (r.kind == 1) cudaMemsetAsync(s->f_dmax, 0, 8, st);
+    if (r.kind == 1) cudaMemsetAsync(f.dmax, 0, 8, st);
     static_assert(SERVE_NBMAX == 10, "k_serve_finalize is instantiated for the server's batch limit");
     k_serve_finalize<SERVE_NBMAX><<<g, 256, 0, st>>>(tal, r.nbatch, nv, scale, r.kind, e->mass_d.as<double>(),
-                                                     e->rho_vox.as<double>(), (double)r.nper, s->f_dose, s->f_var,
-                                                     s->f_dmax);
+                                                     e->rho_vox.as<double>(), (double)r.nper, f.dose, f.var, f.dmax);
     if ((rc = cuda_check(e, cudaGetLastError(), "k_serve_finalize"))) return rc;
+    if (r.kind == 1) {
+        long seglen = (nv + NSEG - 1) / NSEG;
+        k_seg_count<<<NSEG, 256, 0, st>>>(f.dose, nv, seglen, f.dmax, r.rel, f.cnt);
+        k_seg_scan<<<1, NSEG, 0, st>>>(f.cnt, f.off, f.total);
+        k_seg_write<<<NSEG, 256, 0, st>>>(f.dose, f.var, nv, seglen, f.dmax, r.rel, f.off, f.rows, f.vals, f.vars, nv);
+        if ((rc = cuda_check(e, cudaGetLastError(), "sparse extraction"))) return rc;
+        cudaMemcpyAsync(f.total_h, f.total, 8, cudaMemcpyDeviceToHost, st);
+    }
+    return cuda_check(e, cudaEventRecord(f.ev, st), "finalisation");
+}
+
+// The result of a finalised request into host memory, on a stream of its
+// own: the next request's finalisation runs meanwhile.
+int finalize_collect(omc_server *s, Request &r, omc_server::Fin &f) {
+    omc_engine *e = s->e;
+    cudaStream_t st = s->copy_stream;
+    long nv = e->ph.nvox();
+    int rc = cuda_check(e, cudaEventSynchronize(f.ev), "finalisation");
+    if (rc) return rc;
     if (r.kind == 0) {
         r.dose.resize(nv);
         r.unc.resize(nv);
-        cudaMemcpyAsync(r.dose.data(), s->f_dose, nv * 8, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(r.unc.data(), s->f_var, nv * 8, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(r.dose.data(), f.dose, nv * 8, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(r.unc.data(), f.var, nv * 8, cudaMemcpyDeviceToHost, st);
         return cuda_check(e, cudaStreamSynchronize(st), "finalize beam request");
     }
-    long seglen = (nv + NSEG - 1) / NSEG;
-    k_seg_count<<<NSEG, 256, 0, st>>>(s->f_dose, nv, seglen, s->f_dmax, r.rel, s->f_cnt);
-    k_seg_scan<<<1, NSEG, 0, st>>>(s->f_cnt, s->f_off, s->f_total);
-    k_seg_write<<<NSEG, 256, 0, st>>>(s->f_dose, s->f_var, nv, seglen, s->f_dmax, r.rel, s->f_off, s->f_rows,
-                                       s->f_vals, s->f_vars, nv);
-    if ((rc = cuda_check(e, cudaGetLastError(), "sparse extraction"))) return rc;
-    long long nnz = 0;
-    cudaMemcpyAsync(&nnz, s->f_total, 8, cudaMemcpyDeviceToHost, st);
-    if ((rc = cuda_check(e, cudaStreamSynchronize(st), "sparse count"))) return rc;
+    const size_t nnz = (size_t)*f.total_h;
+    const bool staged = nnz * 20 <= FIN_STAGE;
+    if (staged && nnz) {
+        cudaMemcpyAsync(f.stage, f.vals, nnz * 8, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(f.stage + nnz * 8, f.vars, nnz * 8, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(f.stage + nnz * 16, f.rows, nnz * 4, cudaMemcpyDeviceToHost, st);
+    }
     r.rows.resize(nnz);
     r.vals.resize(nnz);
     r.var.resize(nnz);
-    if (nnz > 0) {
-        cudaMemcpyAsync(r.rows.data(), s->f_rows, nnz * 4, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(r.vals.data(), s->f_vals, nnz * 8, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(r.var.data(), s->f_vars, nnz * 8, cudaMemcpyDeviceToHost, st);
+    if (!staged) {
+        cudaMemcpyAsync(r.rows.data(), f.rows, nnz * 4, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(r.vals.data(), f.vals, nnz * 8, cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(r.var.data(), f.vars, nnz * 8, cudaMemcpyDeviceToHost, st);
     }
-    return cuda_check(e, cudaStreamSynchronize(st), "sparse column");
+    if ((rc = cuda_check(e, cudaStreamSynchronize(st), "sparse column"))) return rc;
+    if (staged && nnz) {
+        std::memcpy(r.vals.data(), f.stage, nnz * 8);
+        std::memcpy(r.var.data(), f.stage + nnz * 8, nnz * 8);
+        std::memcpy(r.rows.data(), f.stage + nnz * 16, nnz * 4);
+    }
+    return OMC_OK;
 }
 
 int admit(omc_server *s) {
@@ -477,26 +535,28 @@ int omc_server_create(omc_engine *e, int64_t mem_budget, int max_requests, uint6
         for (auto &q : free_req) q.kind = -1;
         cudaMemcpyAsync(s->sd->req, free_req.data(), sizeof(ServeReq) * SERVE_MAX, cudaMemcpyHostToDevice, e->stream);
     }
-    size_t fin = (size_t)nv * (8 * 6 + 4) + NSEG * 8 + 64;
-    if ((rc = s->fin.alloc(fin))) return set_err(e, rc, "server finalize allocation failed");
-    double *f = s->fin.as<double>();
-    s->f_sum = f;
-    s->f_sum2 = f + nv;
-    s->f_dose = f + 2 * nv;
-    s->f_var = f + 3 * nv;
-    s->f_vals = f + 4 * nv;
-    s->f_vars = f + 5 * nv;
-    s->f_rows = (int *)(f + 6 * nv);
-    s->f_cnt = s->f_rows + nv;
-    s->f_off = s->f_cnt + NSEG;
-    s->f_dmax = (unsigned long long *)(((uintptr_t)(s->f_off + NSEG) + 15) / 16 * 16);
-    s->f_total = (long long *)(s->f_dmax + 1);
+    const size_t fin1 = ((size_t)nv * (8 * 4 + 4) + NSEG * 8 + 64 + 255) / 256 * 256;
+    if ((rc = s->fin.alloc(2 * fin1))) return set_err(e, rc, "server finalize allocation failed");
+    for (int k = 0; k < 2; k++) {
+        omc_server::Fin &f = s->fbuf[k];
+        double *d = (double *)((char *)s->fin.p + k * fin1);
+        f.dose = d;
+        f.var = d + nv;
+        f.vals = d + 2 * nv;
+        f.vars = d + 3 * nv;
+        f.rows = (int *)(d + 4 * nv);
+        f.cnt = f.rows + nv;
+        f.off = f.cnt + NSEG;
+        f.dmax = (unsigned long long *)(((uintptr_t)(f.off + NSEG) + 15) / 16 * 16);
+        f.total = (long long *)(f.dmax + 1);
+    }
     s->slot_req.assign(s->nslots, -1);
     s->slot_seq.assign(s->nslots, 0);
     {
         // pinned snapshot buffers, their events and the finalisation stream
         size_t per = sizeof(ServeReq) * SERVE_MAX + sizeof(int) * SERVE_MAX + 64 + 8 * sizeof(int);
-        if (cudaHostAlloc(&s->snap_host, 2 * per, cudaHostAllocDefault) != cudaSuccess)
+        const size_t stage0 = (2 * per + 255) / 256 * 256;
+        if (cudaHostAlloc(&s->snap_host, stage0 + 2 * FIN_STAGE + 16, cudaHostAllocDefault) != cudaSuccess)
             return set_err(e, OMC_E_CUDA, "server snapshot allocation failed");
         for (int k = 0; k < 2; k++) {
             char *b = (char *)s->snap_host + k * per;
@@ -506,8 +566,14 @@ int omc_server_create(omc_engine *e, int64_t mem_budget, int max_requests, uint6
             s->snap[k].qc = (int *)(b + sizeof(ServeReq) * SERVE_MAX + sizeof(int) * SERVE_MAX + 64);
             if (cudaEventCreateWithFlags(&s->snap[k].ev, cudaEventDisableTiming) != cudaSuccess)
                 return set_err(e, OMC_E_CUDA, "server snapshot event");
+            omc_server::Fin &f = s->fbuf[k];
+            f.stage = (char *)s->snap_host + stage0 + k * FIN_STAGE;
+            f.total_h = (long long *)((char *)s->snap_host + stage0 + 2 * FIN_STAGE) + k;
+            if (cudaEventCreateWithFlags(&f.ev, cudaEventDisableTiming) != cudaSuccess)
+                return set_err(e, OMC_E_CUDA, "server finalisation event");
         }
-        if (cudaStreamCreateWithFlags(&s->fin_stream, cudaStreamNonBlocking) != cudaSuccess)
+        if (cudaStreamCreateWithFlags(&s->fin_stream, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking) != cudaSuccess)
             return set_err(e, OMC_E_CUDA, "server finalisation stream");
     }
     s->target = std::min<long long>((long long)e->ev->cap / 2, e->ev->inflight);
@@ -659,7 +725,7 @@ static int process_snapshot(omc_server *s, omc_server::Snap &sn) {
     if (sn.seq <= s->drain_seq) s->left = 0;   // taken before the drain emptied the queues
     s->injected = true;
     std::vector<int> keep;
-    bool freed = false;
+    std::vector<int> done;   // slots whose requests are finished
     for (int slot : s->order) {
         Request &r = *s->reqs[s->slot_req[slot]];
         if (sn.seq <= s->slot_seq[slot]) {   // admitted after this snapshot was taken
@@ -670,23 +736,28 @@ static int process_snapshot(omc_server *s, omc_server::Snap &sn) {
         const ServeReq &q = sn.req[slot];
         r.injected = q.next;
         if (q.next < r.nhist) s->injected = false;
-        if (q.next >= r.nhist && sn.live[slot] == 0) {
-            if ((rc = finalize_request(s, r))) return rc;
-            r.state = 2;
-            r.t_done = now_ms();
-            s->completed.push_back(r.id);
-            s->finished++;
-            s->slot_req[slot] = -1;
-            ServeReq fr{};
-            fr.kind = -1;
-            cudaMemcpyAsync(&s->sd->req[slot], &fr, sizeof(fr), cudaMemcpyHostToDevice, e->stream);
-            freed = true;
-        } else {
-            keep.push_back(slot);
-        }
+        if (q.next >= r.nhist && sn.live[slot] == 0) done.push_back(slot);
+        else keep.push_back(slot);
     }
+    // two at a time: the next one's kernels run while one is taken over
+    for (size_t k = 0; k < done.size(); k++) {
+        Request &r = *s->reqs[s->slot_req[done[k]]];
+        if (k == 0 && (rc = finalize_launch(s, r, s->fbuf[0]))) return rc;
+        if (k + 1 < done.size() &&
+            (rc = finalize_launch(s, *s->reqs[s->slot_req[done[k + 1]]], s->fbuf[(k + 1) & 1])))
+            return rc;
+        if ((rc = finalize_collect(s, r, s->fbuf[k & 1]))) return rc;
+        r.state = 2;
+        r.t_done = now_ms();
+        s->completed.push_back(r.id);
+        s->finished++;
+        ServeReq fr{};
+        fr.kind = -1;
+        cudaMemcpyAsync(&s->sd->req[done[k]], &fr, sizeof(fr), cudaMemcpyHostToDevice, e->stream);
+    }
+    for (int slot : done) s->slot_req[slot] = -1;
     sn.seq = 0;
-    if (freed) {
+    if (!done.empty()) {
         s->order = keep;
         int n = (int)s->order.size();
         if (n) cudaMemcpyAsync(s->sd->order, s->order.data(), n * sizeof(int), cudaMemcpyHostToDevice, e->stream);
@@ -803,11 +874,11 @@ int omc_server_release(omc_server *s, int id) {
     Request &r = *s->reqs[id];
     if (r.state < 2) return OMC_E_NOTREADY;
     r.state = 3;
-    std::vector<int32_t>().swap(r.rows);
-    std::vector<double>().swap(r.vals);
-    std::vector<double>().swap(r.var);
-    std::vector<double>().swap(r.dose);
-    std::vector<double>().swap(r.unc);
+    Result<int32_t>().swap(r.rows);
+    Result<double>().swap(r.vals);
+    Result<double>().swap(r.var);
+    Result<double>().swap(r.dose);
+    Result<double>().swap(r.unc);
     return OMC_OK;
 }
 
@@ -821,15 +892,16 @@ int omc_run_beamlets(omc_engine *e, const omc_beamlets *b, int64_t nhist, int nb
     if (nbatch < 2) return set_err(e, OMC_E_ARG, "nbatch must be >= 2");
     cudaSetDevice(e->device);
     int nb = b->nbixels;
-    std::vector<std::vector<int32_t>> cr(nb);
-    std::vector<std::vector<double>> cv(nb), cvar(nb);
+    std::vector<Result<int32_t>> cr(nb);
+    std::vector<Result<double>> cv(nb), cvar(nb);
     double t0 = now_ms();
     long long histories = 0;
     double launches = 0;
     if (mode == OMC_EVENT_FP32) {
         if (nbatch > 10) return set_err(e, OMC_E_RANGE, "the event form supports nbatch <= 10");
         omc_server *s = nullptr;
-        if ((rc = omc_server_create(e, 0, 0, seed, &s))) return rc;
+        // tallies for its columns only
+        if ((rc = omc_server_create(e, 0, std::min(nb, SERVE_MAX), seed, &s))) return rc;
         std::unique_ptr<omc_server, int (*)(omc_server *)> guard(s, omc_server_destroy);
         std::vector<int> ids(nb);
         for (int i = 0; i < nb; i++) {
