@@ -45,16 +45,22 @@ struct PhBin {
 
 // Electron bin for one charge (0 = e-, 1 = e+).  `range` is the CSDA range
 // from the first grid energy to the bin's lower edge, `earr` that edge.
+// What a step reads together lies together, in pieces one load can take.
 template <typename R>
-struct ElBin {
-    PL<R> sig, dedx, tmxs, eta, blcce, q1c, q2c, br1, br2;
+struct alignas(4 * sizeof(R)) ElBin {
+    PL<R> dedx, tmxs, eta, blcce, q1c, q2c;
     R range, earr;
+    PL<R> sig, br1, br2;
 };
 
+// Node of the multiple-scattering surface with its alias node's values in the
+// same 32 bytes (FP32): a look-up is one sector of a table that does not fit
+// in L1, not two one after the other.  u, f and the in-bin slope du (0 with
+// ref_compat) of the node and (a) of its alias; w: the alias threshold.
 template <typename R>
-struct MsE {
-    R u, f, w;
-    int i;
+struct alignas(8 * sizeof(R)) MsE {
+    R u, f, du, w;
+    R ua, fa, dua, pad;
 };
 
 // Per-medium scalars.

@@ -186,10 +186,18 @@ void make_layout(const Tables &t, const Phantom &ph, const Regions &rg, double e
     }
     L.msurf.assign(D_NMS, MsE<R>{});
     for (int i = 0; i < D_NMS; i++) {
-        L.msurf[i].u = (R)t.ums[i];
-        L.msurf[i].f = (R)t.fms[i];
-        L.msurf[i].w = (R)t.wms[i];
-        L.msurf[i].i = t.ims[i];
+        MsE<R> &m = L.msurf[i];
+        // the last node of a row is never drawn: slopes end there
+        auto du = [&](int n) { return ref_compat || n % 32 == 31 ? R(0) : (R)t.ums[n + 1] - (R)t.ums[n]; };
+        const int a = i / 32 * 32 + std::min(std::max((int)t.ims[i], 0), 30);
+        m.u = (R)t.ums[i];
+        m.f = (R)t.fms[i];
+        m.du = du(i);
+        m.w = (R)t.wms[i];
+        m.ua = (R)t.ums[a];
+        m.fa = (R)t.fms[a];
+        m.dua = du(a);
+        m.pad = R(0);
     }
     L.spin.assign(t.spin_rej.begin(), t.spin_rej.end());
     d.b2spin_min = t.b2spin_min; d.dbeta2i = t.dbeta2i; d.espml = t.espml; d.dleneri = t.dleneri;
