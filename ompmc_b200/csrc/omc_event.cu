@@ -74,48 +74,78 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // a block, four blocks an SM.  Measured on the slab beam (1e7 histories):
 // 136.5 -> 105.1 ms, code of the kernel 78 -> 63 KB; a fill to 12 at the top
 // of a step and 10 a pass beat 3 / 10 (111.8), 8 / 8 (108.4), 3 / 13 (108.6).
-constexpr int RING = 16;        // numbers a thread holds: ensure() takes up to RING - 3
-// COLS: threads of the block.
-template <int COLS>
+// COLS: threads of the block.  ROWS: numbers a thread holds; ensure() takes
+// up to ROWS - 3.
+constexpr int RING = 16;
+template <int COLS, int ROWS>
 struct RingStore {
-    float v[RING][COLS];
+    float v[ROWS][COLS];
     uint32_t k0[COLS], k1[COLS];
 };
-template <int COLS>
-__device__ __forceinline__ RingStore<COLS> &ring() {
-    __shared__ RingStore<COLS> r;
-    return r;
+template <int COLS, int ROWS>
+__device__ __forceinline__ RingStore<COLS, ROWS> &ring() {
+    if constexpr (sizeof(RingStore<COLS, ROWS>) > 48 * 1024) {
+        extern __shared__ float ring_shared[];
+        return *reinterpret_cast<RingStore<COLS, ROWS> *>(ring_shared);
+    } else {
+        __shared__ RingStore<COLS, ROWS> r;
+        return r;
+    }
 }
-template <int COLS>
-__device__ __noinline__ void ring_fill(uint32_t block, uint32_t seedw) {
-    RingStore<COLS> &r = ring<COLS>();
-    const int t = threadIdx.x;
+// Block `block` of the stream of column t.
+template <int COLS, int ROWS>
+__device__ __forceinline__ void ring_block(uint32_t block, uint32_t seedw, int t) {
+    RingStore<COLS, ROWS> &r = ring<COLS, ROWS>();
     const U4 b = philox4x32_10(U4{block, seedw, 0x6f6d6321u, 0u}, r.k0[t], r.k1[t]);
-    const int row = (block & (RING / 4 - 1)) * 4;
+    const int row = (block & (ROWS / 4 - 1)) * 4;
     r.v[row][t] = u01f(b.x);
     r.v[row + 1][t] = u01f(b.y);
     r.v[row + 2][t] = u01f(b.z);
     r.v[row + 3][t] = u01f(b.w);
 }
-template <int COLS>
+template <int COLS, int ROWS>
+__device__ __noinline__ void ring_fill(uint32_t block, uint32_t seedw) {
+    ring_block<COLS, ROWS>(block, seedw, threadIdx.x);
+}
+template <int COLS, int ROWS = RING>
 struct RingStream {
     uint32_t seedw, pos, filled;
     __device__ __forceinline__ void init(uint64_t key, uint32_t seed_word, uint32_t position = 0) {
-        ring<COLS>().k0[threadIdx.x] = (uint32_t)key;
-        ring<COLS>().k1[threadIdx.x] = (uint32_t)(key >> 32);
+        ring<COLS, ROWS>().k0[threadIdx.x] = (uint32_t)key;
+        ring<COLS, ROWS>().k1[threadIdx.x] = (uint32_t)(key >> 32);
         seedw = seed_word;
         pos = position;
         filled = position & ~3u;
     }
     __device__ __forceinline__ uint32_t position() const { return pos; }
     __device__ __forceinline__ uint64_t key() const {
-        return ((uint64_t)ring<COLS>().k1[threadIdx.x] << 32) | ring<COLS>().k0[threadIdx.x];
+        return ((uint64_t)ring<COLS, ROWS>().k1[threadIdx.x] << 32) | ring<COLS, ROWS>().k0[threadIdx.x];
     }
     __device__ __forceinline__ void ensure(int n) {
         while ((int)(filled - pos) < n) {
-            ring_fill<COLS>(filled >> 2, seedw);
+            ring_fill<COLS, ROWS>(filled >> 2, seedw);
             filled += 4;
         }
+    }
+    // The whole warp fills the rings of the lanes of `lanes`: ROWS / 4 lanes
+    // a ring and pass.
+    __device__ __forceinline__ void assist(unsigned lanes) {
+        constexpr int PER = ROWS / 4 > 32 ? 32 : ROWS / 4;
+        const int lane = threadIdx.x & 31;
+        for (unsigned m = lanes; m;) {
+            unsigned t = m;
+#pragma unroll
+            for (int q = 0; q < 32 / PER; q++) {
+                if (q < lane / PER) t &= t - 1;
+                m &= m - 1;
+            }
+            const int src = t ? __ffs(t) - 1 : 0;
+            const uint32_t f = __shfl_sync(0xffffffffu, filled, src), at = __shfl_sync(0xffffffffu, pos, src);
+            const uint32_t block = (f >> 2) + lane % PER;
+            if (t && (int)(block * 4 + 4 - at) <= ROWS) ring_block<COLS, ROWS>(block, seedw, (threadIdx.x & ~31) + src);
+        }
+        if (lanes >> lane & 1) filled = (pos + ROWS) & ~3u;
+        __syncwarp();
     }
     // continue at a later position (numbers drawn elsewhere)
     __device__ __forceinline__ void seek(uint32_t p) {
@@ -124,7 +154,7 @@ struct RingStream {
     }
     // the caller has asked for it (ensure)
     __device__ __forceinline__ float uni() {
-        const float v = ring<COLS>().v[pos & (RING - 1)][threadIdx.x];
+        const float v = ring<COLS, ROWS>().v[pos & (ROWS - 1)][threadIdx.x];
         pos++;
         return v;
     }
@@ -133,8 +163,8 @@ template <typename Rng>
 struct IsRing {
     static constexpr bool value = false;
 };
-template <int COLS>
-struct IsRing<RingStream<COLS>> {
+template <int COLS, int ROWS>
+struct IsRing<RingStream<COLS, ROWS>> {
     static constexpr bool value = true;
 };
 
@@ -680,6 +710,14 @@ constexpr int DRAIN_STACK = 48;
 // One block of 512 per SM: up to 128 registers, which keep the step's state
 // out of memory.
 constexpr int DRAIN_BLOCK = 512;
+// The ring of a drain lane, filled by the warp before a turn where few lanes
+// are at work: a lone lane spent 23 % of its step in the generator, one block
+// of four numbers after the other.  A turn draws some 45 numbers.  Water 1e4
+// 4.02 -> 3.65 ms, slab 1e6 24.1 -> 23.3; rings of 64 gave the same, with
+// less L1 left (18 MV on 200^3: 75.3 for 73.1 ms), helping up to 4 lanes a warp less.
+constexpr int DRAIN_RING = 32;
+constexpr int DRAIN_HELPED = 8;
+constexpr size_t DRAIN_SHARED = sizeof(RingStore<DRAIN_BLOCK, DRAIN_RING>);
 constexpr int DRAIN_TSTEPS = 1;               // tstep-loop iterations a turn
 constexpr int DRAIN_POOL = 1 << 18;           // donations per launch; beyond them lanes keep their work
 constexpr int DRAIN_POLLS = 1 << 24;          // looks of an idle block at the pool (1 us each) before it gives up
@@ -782,7 +820,7 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
             uint32_t seedw) {
     constexpr int MAXOUT = SPLIT ? EV_MAXOUT_SPLIT : EV_MAXOUT;
     using R = float;
-    using Rng = RingStream<DRAIN_BLOCK>;
+    using Rng = RingStream<DRAIN_BLOCK, DRAIN_RING>;
     using Env = EvEnv<MAXOUT, R, Rng, STATS>;
     const unsigned full = 0xffffffffu;
     const int np = queue_size(qP), ne = queue_size(qE);
@@ -873,6 +911,14 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
             if (alone) __nanosleep(1000);
         } else {
             idle = 0;
+        }
+        {
+            // few lanes at work: the others fill their rings
+            const unsigned charged = __ballot_sync(full, busy && p.iq != 0);
+            if (charged && __popc(charged) <= DRAIN_HELPED) {
+                g.rng.seedw = seedw;
+                g.rng.assist(charged);
+            }
         }
         const uint64_t pkey = g.rng.key();
         g.nout = 0;
@@ -1308,7 +1354,9 @@ static void size_grids(omc_engine *e, EventStateT<R> &S) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bi, k_electron_interact<R>, S.block, 0);
     S.grid_i = e->sm_count * std::max(1, bi);
     if constexpr (sizeof(R) == 4) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain<false, false>, DRAIN_BLOCK, 0);
+        for (auto k : {k_drain<false, false>, k_drain<false, true>, k_drain<true, false>, k_drain<true, true>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DRAIN_SHARED);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain<false, false>, DRAIN_BLOCK, DRAIN_SHARED);
         S.drain_lanes = e->sm_count * std::max(1, bd) * DRAIN_BLOCK;
     } else {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain64<false>, DRAIN64_BLOCK, 0);
@@ -1535,7 +1583,7 @@ static void launch_drain(omc_engine *e, int iph, long long left, double *tallies
         int *ready = S.drain_ready.template as<int>();
         cudaMemsetAsync(ready, 0, DRAIN_POOL * sizeof(int), e->stream);
         cudaMemsetAsync(&S.ctl_d->drain_head, 0, 4 * sizeof(int), e->stream);
-        kd<<<(int)g, DRAIN_BLOCK, 0, e->stream>>>(D, S.q[iph], S.q[iph + 1], S.q[iph ^ 2], ready, tallies, e->ph.nvox(),
+        kd<<<(int)g, DRAIN_BLOCK, DRAIN_SHARED, e->stream>>>(D, S.q[iph], S.q[iph + 1], S.q[iph ^ 2], ready, tallies, e->ph.nvox(),
                                                   S.ctl_d, seedw);
     }
 }
