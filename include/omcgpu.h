@@ -95,7 +95,7 @@ typedef struct {
                              every kernel (see omc_profile_last) */
     int electron_tsteps;  /* event form: tstep-loop iterations an electron runs
                              per launch before it is re-queued (0 = default: 2,
-                             1 in the FP64 event form) */
+                             1 with nsplit > 1 and in the FP64 event form) */
     int64_t inflight;     /* event form: particles kept in flight (0 = default) */
     int tail_boost;       /* event form: largest factor by which event budgets
                              grow as the queues drain (0 = default 32, 1 = fixed

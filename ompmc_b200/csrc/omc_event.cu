@@ -1379,10 +1379,14 @@ int event_interact_queue(omc_engine *e) { return event_interact_queue_t<float>(e
 // warp that go on together do similar work, but every event costs a round
 // trip through the queue.  FP32: 1 / 2 / 3 iterations 100.3 / 98.4 / 108.1 ms
 // on the slab beam (1e7 histories), 103.8 / 94.4 / 92.9 ms on the 200^3-class
-// 18 MV beam (1e6).
+// 18 MV beam (1e6).  Splitting engines run one: their electron
+// queues are full for most of a run, and the longer events of a warp cost
+// more there than the round trips (1 / 2 iterations: 58.3 / 76.0 ms at nsplit
+// 20 on 69^3 water voxels, 23.9 / 25.3 at 20 on 67^3, 31.0 / 32.0 at 10 on a
+// 84^3 CT; 32.0 / 31.7 on the slab phantom).
 template <typename R>
-static int default_tsteps() {
-    return sizeof(R) == 4 ? 2 : 1;
+static int default_tsteps(int nsplit) {
+    return sizeof(R) == 4 && nsplit <= 1 ? 2 : 1;
 }
 
 template <typename R>
@@ -1398,7 +1402,7 @@ static int event_prepare_t(omc_engine *e) {
     S.block = e->opt.block > 0 ? std::min(EV_MAX_BLOCK, (e->opt.block + 31) / 32 * 32) : 256;
     S.grid = e->sm_count * std::max(1, 2048 / S.block);
     size_grids(e, S);
-    S.tsteps = e->opt.electron_tsteps > 0 ? e->opt.electron_tsteps : default_tsteps<R>();
+    S.tsteps = e->opt.electron_tsteps > 0 ? e->opt.electron_tsteps : default_tsteps<R>(e->opt.nsplit);
     S.boost = e->opt.tail_boost > 0 ? e->opt.tail_boost : 32;
     S.inflight = e->opt.inflight > 0 ? e->opt.inflight : (1LL << 20);
     S.esplit = e->opt.electron_split > 0 ? e->opt.electron_split + D_RM : 0.0;
@@ -1485,7 +1489,7 @@ int event_set_params(omc_engine *e, int tsteps, int boost, long long inflight, i
     }
     auto apply = [&](auto &S) {
         using R = decltype(S.q[0].pos->x);
-        S.tsteps = e->opt.electron_tsteps > 0 ? e->opt.electron_tsteps : default_tsteps<R>();
+        S.tsteps = e->opt.electron_tsteps > 0 ? e->opt.electron_tsteps : default_tsteps<R>(e->opt.nsplit);
         S.boost = e->opt.tail_boost > 0 ? e->opt.tail_boost : 32;
         S.inflight = e->opt.inflight > 0 ? e->opt.inflight : (1LL << 20);
         S.esplit = e->opt.electron_split > 0 ? e->opt.electron_split + D_RM : 0.0;
