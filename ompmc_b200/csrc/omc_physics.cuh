@@ -75,6 +75,15 @@ OMC_HD float m_mul(float a, float b) {
     return a * b;
 #endif
 }
+// A sum into which no product before it is contracted.
+OMC_HD double m_add(double a, double b) { return a + b; }
+OMC_HD float m_add(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
 // Sums of products in the electron step, with the product that is
 // contracted into the sum said explicitly: which one the compiler picks
 // depends on the code around, and every FP32 kernel has to round a
@@ -1498,15 +1507,29 @@ OMC_HD R msdist(const DevData<R> &D, Env &g, const Part<R> &p, int imed, int iq,
 // Path length from ekei down to ekef inside one interval of the log-linear
 // stopping-power table (computeDrange, ompmc.c:3997-4033).
 template <typename R>
-OMC_OUTLINE R drange(const DevData<R> &D, int imed, int qel, int lelke, R ekei, R ekef, R elkei, R elkef) {
+OMC_HD R drange_in(const DevData<R> &D, int imed, int qel, int lelke, R ekei, R ekef, R elkei, R elkef) {
     R fedep = R(1) - ekef / ekei;
-    R elktmp = R(0.5) * (elkei + elkef + R(0.25) * fedep * fedep * (R(1) + fedep * (R(1) + R(0.875) * fedep)));
+    R elktmp = R(0.5) * (m_add(elkei, elkef) + R(0.25) * fedep * fedep * (R(1) + fedep * (R(1) + R(0.875) * fedep)));
     const ElBin<R> &B = ebin(D, imed, qel, lelke);
     R dedxmid = pwl(B.dedx, elktmp);
     dedxmid = R(1) / dedxmid;
     R aux = B.dedx.a1 * dedxmid;
     aux = aux * (R(1) + R(2) * aux) * fedep * fedep / (R(6) * (R(2) - fedep) * (R(2) - fedep));
-    return fedep * ekei * dedxmid * (R(1) + aux);
+    return m_mul(fedep * ekei * dedxmid, R(1) + aux);
+}
+
+template <typename R>
+OMC_OUTLINE R drange_out(const DevData<R> &D, int imed, int qel, int lelke, R ekei, R ekef, R elkei, R elkef) {
+    return drange_in(D, imed, qel, lelke, ekei, ekef, elkei, elkef);
+}
+// FP32: in place, so that its table reads and the step's overlap (18 MV on
+// 200^3 voxels 73.9 -> 72.6 ms, slab beam of 1e6 histories 23.5 -> 22.8), the
+// sum of its arguments and its last product rounded as a call's are.  FP64: a
+// call.
+template <typename R>
+OMC_HD R drange(const DevData<R> &D, int imed, int qel, int lelke, R ekei, R ekef, R elkei, R elkef) {
+    if constexpr (sizeof(R) == 4) return drange_in(D, imed, qel, lelke, ekei, ekef, elkei, elkef);
+    else return drange_out(D, imed, qel, lelke, ekei, ekef, elkei, elkef);
 }
 
 // Energy lost to sub-threshold processes over path tustep (computeEloss,
