@@ -37,7 +37,7 @@ SPACE = {
     "block": [64, 128, 256],
     "electron_split": [0.0, 0.1, 0.15, 0.2, 0.3, 0.5, 1.0],
     "electron_chsteps": [1, 2, 3, 4, 8],
-    "drain_particles": [-1, 10000, 20000, 40000, 80000],
+    "drain_particles": [-1, 10000, 20000, 40000, 80000, 114000],
 }
 # the starting point: the best setting measured on the slab workload
 DEFAULT = {"electron_tsteps": 1, "tail_boost": 32, "inflight": 1 << 21, "block": 256, "electron_split": 0.0,

@@ -14,7 +14,8 @@
 //               instruction cache: 8 % faster on slab64)
 // Queues are double-buffered (A -> B, then B -> A), so two cycles form an
 // idempotent CUDA graph that the host replays until every history is
-// injected and few particles are left; k_drain then runs those to the end.
+// injected (after that, one without k_source) and few particles are left;
+// k_drain then runs those to the end.
 //
 // An event transports its particle until the next interaction, death or,
 // for electrons, the end of the cycle's budget of tstep-loop iterations.
@@ -1586,7 +1587,7 @@ static void launch_drain(omc_engine *e, int iph, long long left, double *tallies
         // the pool: the photon output queue, empty between cycles, and its flags
         int *ready = S.drain_ready.template as<int>();
         cudaMemsetAsync(ready, 0, DRAIN_POOL * sizeof(int), e->stream);
-        cudaMemsetAsync(&S.ctl_d->drain_head, 0, 4 * sizeof(int), e->stream);
+        cudaMemsetAsync(&S.ctl_d->drain_head, 0, 3 * sizeof(int), e->stream);
         kd<<<(int)g, DRAIN_BLOCK, DRAIN_SHARED, e->stream>>>(D, S.q[iph], S.q[iph + 1], S.q[iph ^ 2], ready, tallies, e->ph.nvox(),
                                                   S.ctl_d, seedw);
     }

@@ -64,10 +64,9 @@ struct Ctl {
     // drain: the largest sub-history one thread ran (events, events of the
     // particle it started from, transport steps)
     int drain_max_events, drain_max_chain, drain_max_steps, drain_pad;
-    // drain: queued particles taken, particles donated to the pool, taken
-    // from it, tasks done (one 16-byte load)
-    alignas(16) int drain_head;
-    int drain_tail, drain_over, drain_done;
+    // drain: tickets drawn (queued particles taken, then pool entries waited
+    // for), particles put into the pool, tasks done
+    int drain_head, drain_tail, drain_done;
 };
 
 // Per-kernel profile of the last run made with options.profile = 1.
