@@ -354,6 +354,12 @@ int omc_replay(omc_engine *e, const double *prim, int nhist, const double *rn, c
 int omc_kat(omc_engine *e, int which, const double *q, const double *extra, int n, const double *rn,
             const int64_t *rn_off, double *out, int32_t *nout, int64_t *used, uint32_t *flags);
 
+/* Looks that an idle block of the event form's FP32 drain takes, about a
+ * microsecond each, while no particle's sub-history ends anywhere before it
+ * gives up and the run or the server step returns OMC_E_DEVICE (0 = default,
+ * 2^24); tests lower it. */
+int omc_drain_polls(omc_engine *e, int polls);
+
 /* Device allocations (cudaMalloc) the library has made in this process, all
  * engines and devices together; no reference counterpart.  Tests read it
  * around a call to show that the call allocated nothing. */

@@ -181,6 +181,7 @@ enum DevErr : unsigned {
     ERR_LOG = 16u,           // deposit log full
     ERR_LAMBDA = 32u,        // BCA lambda_max <= 0; particle dropped (as the reference)
     ERR_NAN = 64u,           // non-finite state; particle dropped
+    ERR_DRAIN = 128u,        // a block of the drain gave up waiting for work: particles may be left undone
 };
 
 }  // namespace omc

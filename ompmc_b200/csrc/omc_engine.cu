@@ -684,6 +684,12 @@ int omc_event_params(omc_engine *e, int electron_tsteps, int tail_boost, int64_t
     return event_set_params(e, electron_tsteps, tail_boost, (long long)inflight, block, electron_split);
 }
 
+int omc_drain_polls(omc_engine *e, int polls) {
+    if (!e || polls < 0) return global_err(OMC_E_ARG, "omc_drain_polls: bad argument");
+    e->drain_polls = polls;
+    return OMC_OK;
+}
+
 int omc_profile_last(const omc_engine *e, double *out, int n) {
     if (!e || !out || n < 28) return global_err(OMC_E_ARG, "omc_profile_last: bad argument");
     for (int i = 0; i < 28; i++) out[i] = 0;
@@ -806,6 +812,8 @@ int omc_run_beam(omc_engine *e, const omc_beam *b, int64_t ncase, int nbatch, ui
         stats[4] = accum[1];
         stats[5] = (double)ks.flags;
     }
+    if (ks.flags & ERR_DRAIN)
+        return set_err(e, OMC_E_DEVICE, "the drain gave up waiting for work (particles may be left undone)");
     if (ks.flags & (ERR_STACK | ERR_QUEUE | ERR_NAN))
         return set_err(e, OMC_E_DEVICE, "device error flags " + std::to_string(ks.flags) + " (particles dropped)");
     return OMC_OK;

@@ -81,6 +81,7 @@ struct omc_engine {
     omc_options opt{};
     int device = 0;
     int sm_count = 0;
+    int drain_polls = 0;    // looks an idle block of the drain takes without progress (0: DRAIN_POLLS)
     cudaStream_t stream = nullptr;
     omc::DevSet<double> d64;
     omc::DevSet<float> d32;

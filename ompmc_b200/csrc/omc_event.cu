@@ -614,7 +614,7 @@ constexpr int DRAIN_HELPED = 8;
 constexpr size_t DRAIN_SHARED = sizeof(RingStore<DRAIN_BLOCK, DRAIN_RING>);
 constexpr int DRAIN_TSTEPS = 1;               // tstep-loop iterations a turn
 constexpr int DRAIN_POOL = 1 << 18;           // donations per launch; beyond them lanes keep their work
-constexpr int DRAIN_POLLS = 1 << 24;          // looks of an idle block at the pool (1 us each) before it gives up
+constexpr int DRAIN_POLLS = 1 << 24;          // looks of an idle block (1 us each) while no task ends before it gives up
 
 template <typename R>
 struct DrainPart {
@@ -711,7 +711,7 @@ __device__ __noinline__ ElectronEventOut<R, Rng, STATS> electron_event_outline(c
 template <bool SPLIT, bool STATS = false>
 __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
     k_drain(DevData<float> D, Queue qP, Queue qE, Queue pool, int *ready, double *tallies, long nvox, Ctl *ctl,
-            uint32_t seedw) {
+            uint32_t seedw, int polls) {
     constexpr int MAXOUT = SPLIT ? EV_MAXOUT_SPLIT : EV_MAXOUT;
     using R = float;
     using Rng = RingStream<DRAIN_BLOCK, DRAIN_RING>;
@@ -747,7 +747,8 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
         __threadfence();
         *(volatile int *)&ready[k] = 1;
     };
-    for (int idle = 0;;) {
+    int idle = 0, seen = -1;                  // thread 0: looks since a task ended, tasks done then
+    for (;;) {
         // the warps of a block take their iterations, and the phases of an
         // iteration, together, so that they share the instructions they fetch
         const bool block_busy = __syncthreads_or(busy);
@@ -790,18 +791,18 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
             // is left who could make more.
             int over = 0;
             if (threadIdx.x == 0) {
-                over = ld_volatile(&ctl->drain_done) >= n + min(ld_volatile(&ctl->drain_tail), pool_cap);
-                if (over) {
-                    const int done = ld_volatile(&ctl->drain_done);
-                    __threadfence();
-                    over = done >= n + min(ld_volatile(&ctl->drain_tail), pool_cap);
+                const int done = ld_volatile(&ctl->drain_done);
+                __threadfence();
+                over = done >= n + min(ld_volatile(&ctl->drain_tail), pool_cap);
+                idle = done == seen ? idle + 1 : 0;
+                seen = done;
+                if (!over && idle > polls) {
+                    // its tickets may still be given particles: the run fails
+                    atomicOr(&ctl->flags, (unsigned)ERR_DRAIN);
+                    over = 1;
                 }
             }
             if (__syncthreads_or(over)) break;
-            if (++idle > DRAIN_POLLS) {
-                if (threadIdx.x == 0) atomicOr(&ctl->flags, (unsigned)ERR_LOOP);
-                break;
-            }
             if (alone) __nanosleep(1000);
         } else {
             idle = 0;
@@ -1482,7 +1483,7 @@ static void launch_drain(omc_engine *e, int iph, long long left, double *tallies
         cudaMemsetAsync(ready, 0, DRAIN_POOL * sizeof(int), e->stream);
         cudaMemsetAsync(&S.ctl_d->drain_head, 0, 3 * sizeof(int), e->stream);
         kd<<<(int)g, DRAIN_BLOCK, DRAIN_SHARED, e->stream>>>(D, S.q[iph], S.q[iph + 1], S.q[iph ^ 2], ready, tallies, e->ph.nvox(),
-                                                  S.ctl_d, seedw);
+                                                  S.ctl_d, seedw, e->drain_polls > 0 ? e->drain_polls : DRAIN_POLLS);
     }
 }
 

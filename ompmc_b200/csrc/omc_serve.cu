@@ -716,7 +716,7 @@ static int process_snapshot(omc_server *s, omc_server::Snap &sn) {
     omc_engine *e = s->e;
     int rc = cuda_check(e, cudaEventSynchronize(sn.ev), "server step");
     if (rc) return rc;
-    if (*sn.flags & (ERR_QUEUE | ERR_NAN | ERR_STACK))
+    if (*sn.flags & (ERR_QUEUE | ERR_NAN | ERR_STACK | ERR_DRAIN))
         return set_err(e, OMC_E_DEVICE, "device error flags " + std::to_string(*sn.flags) + " in serving");
     // a graph ends with a B -> A cycle: the particles are in queues A
     const long long cap = e->ev->cap;

@@ -122,6 +122,7 @@ def lib():
         "omc_trace_rays": ([C.c_void_p, _dp, C.c_int, C.c_int, _dp, _ip, _ip, _ip, _dp], C.c_int),
         "omc_replay": ([C.c_void_p, _dp, C.c_int, _dp, _lp, C.c_int, _ip, _dp, _ip, _lp, _up], C.c_int),
         "omc_device_allocations": ([], C.c_int64),
+        "omc_drain_polls": ([C.c_void_p, C.c_int], C.c_int),
         "omc_kat": ([C.c_void_p, C.c_int, _dp, _dp, C.c_int, _dp, _lp, _dp, _ip, _lp, _up], C.c_int),
         "omc_server_completed": ([C.c_void_p, _ip, C.c_int, C.POINTER(C.c_int)], C.c_int),
         "omc_server_timer": ([C.c_void_p, C.c_int, _dp], C.c_int),
