@@ -1678,10 +1678,13 @@ OMC_HD int electron_transport(const DevData<R> &D, Env &g, Part<R> &p, R &edep_e
     R ustep = 0;
     int guard = 0;
     for (;;) {  // tstep loop
-        // The top of the tstep loop carries no state but the particle
-        // (demfp is re-drawn here), so an event can stop after a budget of
-        // iterations and resume in a later launch exactly where it was.
-        if (!g.tstep_take()) return E_ALIVE;
+        // In a medium the top of the tstep loop carries no state but the
+        // particle (demfp is re-drawn here), so an event can stop after a
+        // budget of iterations and resume in a later launch exactly where it
+        // was.  In vacuum it carries the medium that the particle came from:
+        // back in it, the loop goes on to the interaction test below (as the
+        // reference's does), so an event is not cut before it gets there.
+        if (!g.tstep_take() && imed != -1) return E_ALIVE;
         rng_ensure(g, 1);
         bool compute_tstep = true;
         R eke = eie - RMr;
