@@ -217,9 +217,9 @@ typedef struct {
  * stats (may be NULL) receives [0] histories run, [1] device seconds of the
  * transport, [2] kernel launches, [3] deposited energy (MeV), [4] source
  * energy (MeV), [5] error flags.  The engine keeps the run's device
- * buffers (tallies, sums, outputs; event form: nbatch*nvox batch tallies)
- * between calls, so repeated runs allocate nothing; they are released
- * with the engine. */
+ * buffers (sums, outputs and nbatch*nvox batch tallies, in the plain form
+ * those of as many batches as fit 1 GB) between calls, so repeated runs
+ * allocate nothing; they are released with the engine. */
 int omc_run_beam(omc_engine *e, const omc_beam *b, int64_t ncase, int nbatch, uint64_t seed, int mode,
                  double *dose, double *unc, double *stats);
 

@@ -59,6 +59,17 @@ int cuda_check(omc_engine *e, cudaError_t rc, const char *what) {
 // Batch tallies of a plain run held at once, at most (bytes).
 constexpr long PLAIN_TALLIES = 1L << 30;
 
+int plain_tallies(DBuf &work, int nbatch, long nv, int &group) {
+    group = (int)std::max<long>(1, std::min<long>(nbatch, PLAIN_TALLIES / (nv * 8)));
+    int rc = work.reserve((size_t)group * nv * 8);
+    if (rc == OMC_E_NOMEM && group > 1) {
+        cudaGetLastError();
+        group = 1;
+        rc = work.reserve((size_t)nv * 8);
+    }
+    return rc;
+}
+
 template <typename T>
 static int upload(omc_engine *e, DBuf &b, const std::vector<T> &v) {
     int rc = b.alloc(v.size() * sizeof(T));
@@ -755,15 +766,9 @@ int omc_run_beam(omc_engine *e, const omc_beam *b, int64_t ncase, int nbatch, ui
         BeamSrc<double> S = beam_setup<double>(e, b);
         S.cdf1 = ncdf > 0 ? cdf.as<double>() : nullptr;
         S.cdf2 = ncdf > 0 ? cdf.as<double>() + ncdf : nullptr;
-        // batches run together, each on a tally of its own, as many as fit
-        // PLAIN_TALLIES bytes (one at a time where not even that can be had)
-        DBuf &work = e->run_work;
-        int group = (int)std::max<long>(1, std::min<long>(nbatch, PLAIN_TALLIES / (nv * 8)));
-        while ((rc = work.reserve((size_t)group * nv * 8)) == OMC_E_NOMEM && group > 1) {
-            cudaGetLastError();
-            group = 1;
-        }
-        if (rc) return set_err(e, rc, "device allocation for tallies failed");
+        DBuf &work = e->run_tal;
+        int group;
+        if ((rc = plain_tallies(work, nbatch, nv, group))) return set_err(e, rc, "device allocation for tallies failed");
         cudaMemsetAsync(work.p, 0, (size_t)group * nv * 8, e->stream);
         int block = e->opt.block > 0 ? e->opt.block : 128;
         cudaEvent_t t0, t1;

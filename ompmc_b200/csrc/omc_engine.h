@@ -93,7 +93,7 @@ struct omc_engine {
     void *result_stage = nullptr;   // pinned buffers large results pass through
     // device buffers of omc_run_beam, kept between calls and grown on
     // demand so that a run allocates nothing once the engine is warm
-    omc::DBuf run_sum, run_sum2, run_out, run_unc, run_acc, run_cdf, run_work, run_tal, run_cdf32;
+    omc::DBuf run_sum, run_sum2, run_out, run_unc, run_acc, run_cdf, run_tal, run_cdf32;
 };
 
 namespace omc {
@@ -104,10 +104,13 @@ int cuda_check(omc_engine *e, cudaError_t rc, const char *what);
 // history hist0 on, batch k tallied at work + k * nvox, in launches of at
 // most a few million histories (*launches, may be null, counts them).
 // `next` is a work counter in device memory.
+// Tallies for `group` batches that run together: as many of nbatch as fit 1 GB,
+// one at a time where there is no memory for them.
+int plain_tallies(DBuf &work, int nbatch, long nv, int &group);
 int plain_beam_batches(omc_engine *e, const BeamSrc<double> &S, double *work, uint64_t seed, long hist0, int nbatch,
                        long nper, unsigned long long *next, double *src_energy, int block, long *launches = nullptr);
 int plain_beamlet_batches(omc_engine *e, const BeamletSrc<double> &S, int ib, double *work, uint64_t seed, long hist0,
-                          int nbatch, long nper, unsigned long long *next, int block);
+                          int nbatch, long nper, unsigned long long *next, int block, long *launches = nullptr);
 int plain_trace(omc_engine *e, const double *rays_d, int nrays, int cap, double *ustep, int *irnew, int *idisc,
                 int *ncalls, double *hn);
 // `stacks`: plain_replay_stack_bytes(nhist) of device memory for the

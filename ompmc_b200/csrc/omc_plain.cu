@@ -424,9 +424,9 @@ int plain_beam_batches(omc_engine *e, const BeamSrc<double> &S, double *work, ui
 }
 
 int plain_beamlet_batches(omc_engine *e, const BeamletSrc<double> &S, int ib, double *work, uint64_t seed, long hist0,
-                          int nbatch, long nper, unsigned long long *next, int block) {
+                          int nbatch, long nper, unsigned long long *next, int block, long *launches) {
     auto kernel = e->d64.d.nsplit > 1 ? k_plain_beamlet<SPLIT_STACK> : k_plain_beamlet<PLAIN_STACK>;
-    return plain_chunks(e, nbatch * nper, next, nullptr, "k_plain_beamlet launch", [&](long h0, long n) {
+    return plain_chunks(e, nbatch * nper, next, launches, "k_plain_beamlet launch", [&](long h0, long n) {
         int width;
         const int grid = plain_grid(e, kernel, block, n, width);
         kernel<<<grid, block, 0, e->stream>>>(e->d64.d, S, ib, work, e->ph.nvox(), seed, hist0, h0, n, nper, width,

@@ -928,10 +928,9 @@ int omc_run_beamlets(omc_engine *e, const omc_beamlets *b, int64_t nhist, int nb
         if ((rc = upload_plan<double>(e, b, pb.f64, pb.s64))) return rc;
         long nv = e->ph.nvox();
         DBuf work, fin;
-        const int group = (int)std::max<long>(1, std::min<long>(nbatch, (1L << 30) / (nv * 8)));   // batches run together
-        if ((rc = work.alloc((size_t)group * nv * 8))) return set_err(e, rc, "alloc");
         size_t finb = (size_t)nv * (8 * 6 + 4) + NSEG * 8 + 64;
-        if ((rc = fin.alloc(finb))) return set_err(e, rc, "alloc");
+        int group;
+        if ((rc = fin.alloc(finb)) || (rc = plain_tallies(work, nbatch, nv, group))) return set_err(e, rc, "alloc");
         cudaMemsetAsync(work.p, 0, (size_t)group * nv * 8, e->stream);
         double *f = fin.as<double>();
         double *sum = f, *sum2 = f + nv, *dose = f + 2 * nv, *vv = f + 3 * nv, *fvals = f + 4 * nv, *fvars = f + 5 * nv;
@@ -950,9 +949,11 @@ int omc_run_beamlets(omc_engine *e, const omc_beamlets *b, int64_t nhist, int nb
             if (!e->opt.ref_compat) cudaMemsetAsync(sum2, 0, nv * 8, e->stream);
             for (int b0 = 0; b0 < nbatch; b0 += group) {
                 const int nbt = std::min(group, nbatch - b0);
+                long nl = 0;
                 if ((rc = plain_beamlet_batches(e, pb.s64, i, work.as<double>(), seed, (long)b0 * nper, nbt, nper, next,
-                                                block)))
+                                                block, &nl)))
                     return rc;
+                launches += (double)(nl + 1);
                 if ((rc = fold(e, work.as<double>(), nbt, sum, sum2, nv, 1.0 / (double)nper))) return rc;
             }
             if ((rc = finalize_matrad(e, sum, sum2, nbatch, dose, vv))) return rc;
@@ -976,7 +977,7 @@ int omc_run_beamlets(omc_engine *e, const omc_beamlets *b, int64_t nhist, int nb
                 cudaMemcpy(cvar[i].data(), fvars, n * 8, cudaMemcpyDeviceToHost);
             }
             histories += (long long)nper * nbatch;
-            launches += 2.0 * nbatch + 5;
+            launches += 5;
         }
         unsigned flags = 0;
         cudaMemcpy(&flags, e->errword.p, sizeof(unsigned), cudaMemcpyDeviceToHost);
