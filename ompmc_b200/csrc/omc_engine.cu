@@ -7,11 +7,10 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <system_error>
-#include <thread>
 
 #include "omc_engine.h"
 #include "omc_event.h"
+#include "omc_stripes.h"
 
 using namespace omc;
 
@@ -458,15 +457,7 @@ int fetch_result(omc_engine *e, void *dst, const void *src, size_t bytes) {
             if (x) cudaEventDestroy(x);
         if (rc != cudaSuccess) failed = (int)rc;
     };
-    std::vector<std::thread> pool;
-    int rest = 1;   // stripes that have no thread are done here, after our own
-    try {
-        for (; rest < RESULT_THREADS; rest++) pool.emplace_back(work, rest);
-    } catch (const std::system_error &) {
-    }
-    work(0);
-    for (; rest < RESULT_THREADS; rest++) work(rest);
-    for (auto &t : pool) t.join();
+    run_stripes(RESULT_THREADS, work);
     return failed ? cuda_check(e, (cudaError_t)(int)failed, "d2h") : OMC_OK;
 }
 }  // namespace
