@@ -1908,7 +1908,7 @@ void serve_profile_reset(omc_engine *e) {
 // queues are emptied and every request's live count is zero.
 void serve_drain(omc_engine *e, ServeDev *sd, long long left, double *tallies) {
     EventState &S = *e->ev;
-    launch_drain(e, 0, left, tallies, SERVE_SEEDW);
+    launch_drain(e, 0, left, tallies, SERVE_SEEDW, e->opt.profile != 0);
     cudaMemsetAsync(sd->live, 0, sizeof(sd->live), e->stream);
     cudaMemsetAsync(S.ctl_d->cnt, 0, 2 * sizeof(int), e->stream);
     cudaMemsetAsync(S.ctl_d->cnt_hi, 0, 2 * sizeof(int), e->stream);
