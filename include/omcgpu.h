@@ -290,9 +290,12 @@ int omc_server_submit_beamlet(omc_server *s, const omc_beamlets *b, int ibixel, 
                               double rel_threshold, uint64_t seed);
 int omc_server_submit_beam(omc_server *s, const omc_beam *b, int64_t nhist, int nbatch, uint64_t seed);
 /* Advances the device by up to `cycles` transport cycles, or, when nothing
- * is pending, every running request is fully injected and at most the
- * engine's drain_particles are left, by one drain launch that runs them to
- * the end; *active receives the requests still running. */
+ * is pending and at most the engine's drain_particles are left, by one drain
+ * launch that runs them to the end (histories still to be injected count as
+ * left, and two cycles inject them first; engines with photon splitting wait
+ * until all are injected).  The step after a drain launches nothing unless a
+ * request was admitted since: it finishes the drained ones.  *active receives
+ * the requests still running. */
 int omc_server_step(omc_server *s, int cycles, int *active);
 /* Status of a request: OMC_OK when finished, OMC_E_NOTREADY while running. */
 int omc_server_poll(omc_server *s, int id, double *latency_ms);

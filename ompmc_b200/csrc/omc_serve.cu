@@ -776,7 +776,12 @@ int omc_server_step(omc_server *s, int cycles, int *active) {
     int rc = admit(s);
     if (rc) return rc;
     const int prev = s->cur ^ 1;
-    if (!s->order.empty()) {
+    // The last step's work was a drain and nothing has been admitted since: all
+    // that was injected is done, so its snapshot is looked at before more is
+    // launched (profiled servers read their counters with the next cycle).
+    bool settle = s->snap[prev].seq > 0 && s->snap[prev].seq == s->drain_seq + 1 && !e->opt.profile;
+    for (int slot : s->order) settle = settle && s->slot_seq[slot] < s->snap[prev].seq;
+    if (!s->order.empty() && !settle) {
         const long long dthr = drain_threshold(e);
         const int per_cycle = e->d32.d.defer_interact ? 5 : 4;
         // what the drain would have to run, histories to inject included
