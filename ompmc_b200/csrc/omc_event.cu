@@ -182,14 +182,12 @@ __device__ __forceinline__ void qload(const Queue &q, int i, Part<float> &p, int
     k0 = c.z; k1 = c.w;
 }
 
-template <bool SHARED = false>
 __device__ __forceinline__ void qload(const QueueT<double> &q, int i, Part<double> &p, int &tag, uint32_t &k0,
                                       uint32_t &k1, uint32_t &ctr) {
     const double2 *pa = (const double2 *)&q.pos[i], *pb = (const double2 *)&q.dir[i];
-    const double2 a0 = qread<SHARED>(pa), a1 = qread<SHARED>(pa + 1), b0 = qread<SHARED>(pb),
-                  b1 = qread<SHARED>(pb + 1);
-    const uint4 c = qread<SHARED>(&q.id[i]);
-    ctr = qread<SHARED>(&q.ctr[i]);
+    const double2 a0 = __ldcs(pa), a1 = __ldcs(pa + 1), b0 = __ldcs(pb), b1 = __ldcs(pb + 1);
+    const uint4 c = __ldcs(&q.id[i]);
+    ctr = __ldcs(&q.ctr[i]);
     p.x = a0.x; p.y = a0.y; p.z = a1.x; p.u = a1.y;
     p.v = b0.x; p.w = b0.y; p.e = b1.x; p.wt = b1.y;
     p.ir = (int)c.x;
@@ -981,9 +979,8 @@ __global__ void __launch_bounds__(DRAIN_BLOCK, 1)
 // The FP64 event form's drain: one thread per queued particle in order, with
 // its secondaries on the local stack.  FP64 rounding is the compiler's choice
 // kernel by kernel, and the accuracy study's results rest on this one's.
-// STATS (profiled runs): record the largest sub-history a thread ran.
 constexpr int DRAIN64_BLOCK = 128;
-template <bool STATS = false, typename R = double>
+template <typename R = double>
 __global__ void __launch_bounds__(DRAIN64_BLOCK, 4) k_drain64(DevData<R> D, QueueT<R> qP, QueueT<R> qE, double *tallies,
                                                           long nvox, Ctl *ctl, uint32_t seedw) {
     constexpr int MAXOUT = EV_MAXOUT;
@@ -1007,13 +1004,7 @@ __global__ void __launch_bounds__(DRAIN64_BLOCK, 4) k_drain64(DevData<R> D, Queu
         g.flags = 0;
         g.natom = 0;
         int top = 0;
-        // this sub-history: events, events of its first particle, steps
-        int x_ev = 0, x_chain = 0, x_steps = 0;
-        bool first_alive = true;
         for (int guard = 0; top >= 0; guard++) {
-            const bool first = first_alive && top == 0;
-            x_ev++;
-            x_chain += first;
             if (guard > (1 << 22)) {
                 g.flags |= ERR_LOOP;
                 break;
@@ -1031,7 +1022,6 @@ __global__ void __launch_bounds__(DRAIN64_BLOCK, 4) k_drain64(DevData<R> D, Queu
             if (kind == 1) alive = electron_step<R, EvEnv<MAXOUT, R>, false>(D, g, p) == E_ALIVE;
             else alive = photon_event(D, g, p);
             c_ev[kind]++;
-            x_steps += g.work;
             c_steps[kind] += g.work;
             c_cross[kind] += g.ncross;
             c_dep[kind] += g.ndep;
@@ -1045,7 +1035,6 @@ __global__ void __launch_bounds__(DRAIN64_BLOCK, 4) k_drain64(DevData<R> D, Queu
                 e.pos = g.rng.position();
             } else {
                 top--;
-                first_alive = first_alive && !first;
             }
             for (int k = 0; k < g.nout; k++) {
                 const Part<R> &s2 = g.out[k];
@@ -1068,11 +1057,6 @@ __global__ void __launch_bounds__(DRAIN64_BLOCK, 4) k_drain64(DevData<R> D, Queu
             }
         }
         g.flush();
-        if (STATS) {
-            atomicMax(&ctl->drain_max_events, x_ev);
-            atomicMax(&ctl->drain_max_chain, x_chain);
-            atomicMax(&ctl->drain_max_steps, x_steps);
-        }
         c_atom[1] += g.natom;     // tally atomics of the whole sub-history
         flags |= g.flags;
     }
@@ -1254,7 +1238,7 @@ static void size_grids(omc_engine *e, EventStateT<R> &S) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain<false, false>, DRAIN_BLOCK, DRAIN_SHARED);
         S.drain_lanes = e->sm_count * std::max(1, bd) * DRAIN_BLOCK;
     } else {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain64<false>, DRAIN64_BLOCK, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bd, k_drain64<double>, DRAIN64_BLOCK, 0);
         S.drain_lanes = e->sm_count * std::max(1, bd) * DRAIN64_BLOCK;
     }
     S.lanes = S.grid_e * S.block;
@@ -1470,8 +1454,7 @@ static void launch_drain(omc_engine *e, int iph, long long left, double *tallies
     if constexpr (sizeof(R) == 8) {
         const long long g = std::max(1LL, std::min((left + DRAIN64_BLOCK - 1) / DRAIN64_BLOCK,
                                                    (long long)S.drain_lanes / DRAIN64_BLOCK * 4));
-        auto kd = stats ? k_drain64<true> : k_drain64<false>;
-        kd<<<(int)g, DRAIN64_BLOCK, 0, e->stream>>>(D, S.q[iph], S.q[iph + 1], tallies, e->ph.nvox(), S.ctl_d, seedw);
+        k_drain64<double><<<(int)g, DRAIN64_BLOCK, 0, e->stream>>>(D, S.q[iph], S.q[iph + 1], tallies, e->ph.nvox(), S.ctl_d, seedw);
     } else {
         // a warp per particle, up to one wave of resident blocks
         const long long warps = DRAIN_BLOCK / 32;
