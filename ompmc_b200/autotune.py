@@ -37,11 +37,11 @@ SPACE = {
     "block": [64, 128, 256],
     "electron_split": [0.0, 0.1, 0.15, 0.2, 0.3, 0.5, 1.0],
     "electron_chsteps": [1, 2, 3, 4, 8],
-    "drain_particles": [-1, 10000, 20000, 40000, 80000, 114000],
+    "drain_particles": [-1, 0, 10000, 20000, 40000, 80000],   # 0: the engine's own, from its resident threads
 }
-# the starting point: the best setting measured on the slab workload
-DEFAULT = {"electron_tsteps": 1, "tail_boost": 32, "inflight": 1 << 21, "block": 256, "electron_split": 0.0,
-           "electron_chsteps": 3, "drain_particles": 40000}
+# the starting point: what an engine without photon splitting runs by default
+DEFAULT = {"electron_tsteps": 2, "tail_boost": 32, "inflight": 1 << 20, "block": 256, "electron_split": 0.0,
+           "electron_chsteps": 3, "drain_particles": 0}
 
 
 def _rate(eng, cfg, nhist, run_kw, repeats):
