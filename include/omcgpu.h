@@ -125,7 +125,9 @@ typedef struct {
                              launch instead of further cycles (0 = default,
                              one and a half times the drain kernel's resident
                              threads, once them when photons are split, half
-                             of them in the FP64 event form; -1 = never);
+                             of them in the FP64 event form; -1 = never; runs
+                             of more split photons than it holds at once wait
+                             nsplit cycles after the last injection);
                              results do not depend on it */
 } omc_options;
 

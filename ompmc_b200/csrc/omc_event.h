@@ -172,6 +172,8 @@ void serve_profile_reset(omc_engine *e);
 // Particles left at or below which a run whose histories are all injected
 // switches from transport cycles to the drain kernel (0: never).
 long long drain_threshold(const omc_engine *e);
+// Cycles it waits for after the last of `histories` has been injected.
+long split_cycles(const omc_engine *e, long long histories);
 PlanCfg plan_cfg(const omc_engine *e, long long target);
 int event_set_params(omc_engine *e, int tsteps, int boost, long long inflight, int block, double split_kinetic);
 

@@ -336,6 +336,7 @@ struct omc_server {
     int cur = 0;
     long long seq = 0;               // snapshots taken so far
     long long drain_seq = -1;        // snapshots taken before the last drain
+    long long ripe_from = 0;         // cycles run when the last history may have been injected
     std::vector<long long> slot_seq; // snapshots taken before each slot's admission
     cudaStream_t fin_stream = nullptr;  // finalisation, beside the transport
     ~omc_server() {
@@ -465,6 +466,7 @@ int admit(omc_server *s) {
         s->injected = false;
         s->slot_req[slot] = r.id;
         s->slot_seq[slot] = s->seq;
+        s->ripe_from = s->cycles;
         s->order.push_back(slot);
         ServeReq q{};
         q.kind = r.kind;
@@ -739,6 +741,7 @@ static int process_snapshot(omc_server *s, omc_server::Snap &sn) {
         if (q.next >= r.nhist && sn.live[slot] == 0) done.push_back(slot);
         else keep.push_back(slot);
     }
+    if (!s->injected) s->ripe_from = s->cycles;
     // two at a time: the next one's kernels run while one is taken over
     for (size_t k = 0; k < done.size(); k++) {
         Request &r = *s->reqs[s->slot_req[done[k]]];
@@ -785,8 +788,13 @@ int omc_server_step(omc_server *s, int cycles, int *active) {
         const long long dthr = drain_threshold(e);
         const int per_cycle = e->d32.d.defer_interact ? 5 : 4;
         // what the drain would have to run, histories to inject included
-        long long todo = s->left;
-        for (int slot : s->order) todo += s->reqs[s->slot_req[slot]]->nhist - s->reqs[s->slot_req[slot]]->injected;
+        long long todo = s->left, all = 0;
+        for (int slot : s->order) {
+            const Request &r = *s->reqs[s->slot_req[slot]];
+            todo += r.nhist - r.injected;
+            all += r.nhist;
+        }
+        const bool ripe = s->cycles - s->ripe_from >= split_cycles(e, all);
         const bool ends = dthr > 0 && s->pending.empty() && todo > 0 && todo <= dthr && !e->opt.profile;
         if (ends && !s->injected && e->d32.d.nsplit <= 1) {
             // a load that the drain can hold: two cycles inject all of it, and
@@ -799,7 +807,7 @@ int omc_server_step(omc_server *s, int cycles, int *active) {
             s->drains++;
             s->left = 0;
             s->drain_seq = s->seq;
-        } else if (dthr > 0 && s->injected && s->pending.empty() && s->left > 0 && s->left <= dthr) {
+        } else if (dthr > 0 && s->injected && s->pending.empty() && s->left > 0 && s->left <= dthr && ripe) {
             // the drain's kernel reads the queue sizes on the device; `left`
             // (from the last snapshot, taken before more cycles ran) bounds them
             serve_drain(e, s->sd, s->left, s->tallies.as<double>());
