@@ -594,8 +594,9 @@ __global__ void __launch_bounds__(EV_MAX_BLOCK) k_electron_interact(DevData<R> D
 // an entry has a taker at once; one that a full stack puts there waits for the
 // next warp without work.  The launch is over when as many tasks are
 // done as were made.  Lanes wait only when no particle is left unclaimed, so
-// blocks that are not resident yet hold nobody up, and every wait has a
-// limit.
+// blocks that are not resident yet hold nobody up, and the wait has a limit:
+// a block that finds nothing while no task ends anywhere gives up (ERR_DRAIN),
+// and as its tickets may be given more, the run fails.
 // SPLIT: photons are split rays (nsplit > 1) whose state (next sub-photon,
 // survivor, offset) rides along with them, as in the photon queues.
 constexpr int DRAIN_STACK = 48;
@@ -1258,7 +1259,8 @@ int event_interact_queue(omc_engine *e) { return event_interact_queue_t<float>(e
 // warp that go on together do similar work, but every event costs a round
 // trip through the queue.  FP32: 1 / 2 / 3 iterations 100.3 / 98.4 / 108.1 ms
 // on the slab beam (1e7 histories), 103.8 / 94.4 / 92.9 ms on the 200^3-class
-// 18 MV beam (1e6).  Splitting engines run one: their electron
+// 18 MV beam (1e6); a server whose queues stay full (343 columns of 1.5e5
+// histories) 62.9 / 65.9 M hist/s.  Splitting engines run one: their electron
 // queues are full for most of a run, and the longer events of a warp cost
 // more there than the round trips (1 / 2 iterations: 58.3 / 76.0 ms at nsplit
 // 20 on 69^3 water voxels, 23.9 / 25.3 at 20 on 67^3, 31.0 / 32.0 at 10 on a
@@ -1648,8 +1650,7 @@ int event_run_beam(omc_engine *e, const omc_beam *b, long nper, int nbatch, uint
     } else if (!(rc = capture(0))) {
         // Checked after every graph where the end is near: from the start on
         // when one cycle injects all (with splitting, where the drain's lanes
-        // hold all sub-photons: 10^3 histories split in 20 15.7 -> 11.1 ms, but
-        // 10^4 18.9 -> 26.5).
+        // hold all sub-photons: 10^3 histories split in 20 15.7 -> 11.1 ms).
         const long long few = pweight == 1 ? target : S.drain_lanes;
         int per_check = sizeof(R) == 4 && c0.hist_total * pweight <= few ? 1 : 4;
         for (long graphs = 0;;) {
