@@ -63,3 +63,21 @@ def test_batches_run_one_at_a_time_without_memory():
     # a launch and a fold each for all batches together or for every batch,
     # and five to finish a column
     assert st["launches"] == 2 * (2 + 5) and st1["launches"] == 2 * (2 * BATCHES + 5)
+
+
+@pytest.mark.parametrize("n,histories,nbatch", [(64, 2000, 10), (61, 1501, 7), (20, 3000, 4)])
+def test_batches_of_a_group_keep_apart(n, histories, nbatch):
+    """The batch uncertainty, which a history tallied in another batch than its
+    own would change: all batches in one launch, in launches of three (fixed
+    scratch, 64^3 voxels) and of four or all (smaller grids)."""
+    from ompmc_b200.engine import PLAIN_FP64, Engine
+    ph = cases._phantom("water", n, 300.0 / n)
+    eng = Engine(cases._tables(tuple(ph.media)), ph)
+    call = dict(ncase=histories, nbatch=nbatch, seed=9, mono_energy=4.0, collimator=(-4.0, 4.0, -3.0, 3.0))
+    dose, unc, _ = eng.run_beam(mode=PLAIN_FP64, **call)
+    dose1, unc1, _ = eng.run_beam_noalloc(**call)
+    eng.close()
+    hit = dose > 0
+    assert hit.sum() > 100 and 0 < unc[hit].min() < 0.9
+    np.testing.assert_allclose(dose1, dose, rtol=1e-12)
+    np.testing.assert_allclose(unc1[hit], unc[hit], rtol=1e-6, atol=1e-9)
